@@ -19,20 +19,27 @@ Kinds of cases:
   parallel, fan or Long-Fessler model;
 * ``objective``: cost and gradient of the TV-regularised reconstruction
   (``recon.Objective``), 2D or 3D: what an iteration evaluates;
-* ``unet``: inference of the warm-start network or one training step.
+* ``conv``: one 3x3x3 convolution layer of the warm-start network through the
+  C interface (``include/trtt_b200.h``), at a layer's channels: inference
+  (``trtt_b200_conv3_forward``), or forward, input gradient and weight and bias
+  gradients (``trtt_b200_conv3_wgrad``) as a training step calls them.  The
+  whole network is no case: one BF16 rounding more or less in a layer travels
+  through those behind it, to 1e-3 of the output.
 """
 from __future__ import annotations
 
+import ctypes
 import math
-import os
 
 import numpy as np
 import torch
 
-HERE = os.path.dirname(os.path.abspath(__file__))
-WEIGHTS = os.path.join(os.path.dirname(HERE), "yoricktrtt_b200", "weights", "unet_warmstart_128.npz")
 RSC, RSD = 1000.0, 1500.0  # source to isocentre, source to detector (mm)
 SLOPE = 0.1                # leaky ReLU of the network
+
+# the network's layers: channels of the first and the skip input, output channels
+LAYERS = {"e1a": (16, 0, 16), "e1b": (16, 0, 16), "e2a": (16, 0, 32), "e2b": (32, 0, 32), "e3a": (32, 0, 64),
+          "e3b": (64, 0, 64), "d2a": (64, 32, 32), "d1a": (32, 16, 16)}
 
 
 def listed():
@@ -70,10 +77,11 @@ def listed():
         # Long-Fessler separable footprints on the fan-beam scan
         dict(name="long_fessler_512", kind="pair2d", mode="lf", nx=512, ny=512, nv=1024, views=720, table=0,
              object="phantom", s_scl=0.5, d_scl=0.5),
-        # warm-start network: inference on one volume, and a training step at
-        # the training batch
-        dict(name="unet_infer_128", kind="unet", train=False, batch=1, d=128, h=128, w=128),
-        dict(name="unet_train_64", kind="unet", train=True, batch=2, d=64, h=64, w=64),
+        # warm-start network: the largest layer of an inference at 128^3 (the
+        # decoder's concatenated input at full resolution), and a layer of a
+        # training step at batch 2, half resolution
+        dict(name="conv_infer_128", kind="conv", layer="d1a", train=False, batch=1, d=128, h=128, w=128),
+        dict(name="conv_train_64", kind="conv", layer="e2b", train=True, batch=2, d=64, h=64, w=64),
     ]
 
 
@@ -83,7 +91,7 @@ def _log_int(rng, lo, hi):
 
 def draw(rng):
     kind = rng.choice(["pair3d", "pair3d", "pair3d", "view3d", "gates4d", "pair2d", "pair2d", "objective",
-                       "objective", "unet", "unet"])
+                       "objective", "conv", "conv"])
     if kind in ("pair3d", "view3d", "gates4d") or (kind == "objective" and rng.random() < 0.5):
         n = _log_int(rng, 24, 176)
         square = rng.random() < 0.5
@@ -132,9 +140,9 @@ def draw(rng):
         mode = rng.choice(["parallel", "fan", "fan", "lf"])
         return dict(kind=kind, mode=mode, table=0 if mode == "lf" else rng.choice([0, 10001]),
                     object=rng.choice(["phantom", "iterate"]), **base)
-    d, h, w = (4 * rng.randint(6, 30) for _ in range(3))
-    train = rng.random() < 0.5
-    return dict(kind="unet", train=train, batch=rng.randint(1, 2), d=d, h=h, w=w)
+    d, h, w = (4 * rng.randint(5, 30) for _ in range(3))
+    return dict(kind="conv", layer=rng.choice(sorted(LAYERS)), train=rng.random() < 0.5,
+                batch=rng.randint(1, 2), d=d, h=h, w=w)
 
 
 # ---------------------------------------------------------------------------
@@ -213,12 +221,20 @@ def _gates(case, seed):
 def _inputs(case, seed):
     """Everything random of a case, as GPU tensors and host arrays."""
     k = case["kind"]
-    if k == "unet":
-        n = (case["d"], case["h"], case["w"])
-        target = torch.stack([_ellipsoids(n[2], n[1], n[0], seed * 16 + b) for b in range(case["batch"])])
-        x = torch.nn.functional.avg_pool3d(target[:, None], 3, 1, 1, count_include_pad=False)[:, 0]
-        x = x + 0.03 * torch.randn(x.shape, device="cuda", generator=_gen(seed))
-        return {"x": x.contiguous(), "target": target.contiguous()}
+    if k == "conv":
+        c1, c2, co = LAYERS[case["layer"]]
+        g = _gen(seed)
+
+        def act(c, scale):
+            """Padded channels-last BF16 activations (zero border)."""
+            a = torch.zeros(case["batch"], case["d"] + 2, case["h"] + 2, case["w"] + 2, c, device="cuda")
+            v = a[:, 1:-1, 1:-1, 1:-1]
+            v.copy_(torch.nn.functional.leaky_relu(torch.randn(v.shape, device="cuda", generator=g), SLOPE) * scale)
+            return a.bfloat16()
+
+        w = torch.randn(co, 27, c1 + c2, device="cuda", generator=g) * math.sqrt(2.0 / (27 * (c1 + c2)))
+        return {"x1": act(c1, 0.5), "x2": act(c2, 0.5) if c2 else None, "gy": act(co, 1e-3),
+                "w": w.bfloat16().float(), "b": 0.02 * torch.randn(co, device="cuda", generator=g)}
     if k == "gates4d":
         t, theta = _gates(case, seed)
         vol = torch.stack([_ellipsoids(case["nx"], case["ny"], case["nz"], seed,
@@ -266,14 +282,55 @@ def _projector(case, theta):
                                           len(theta), mode=mode, rsc=RSC, rsd=RSD, theta=theta), table)
 
 
+def _ptr(t):
+    return None if t is None else ctypes.c_void_p(t.data_ptr())
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _prepare_conv(case, s):
+    """Packed weights, output and gradient buffers and scratch, as the network keeps them."""
+    from yoricktrtt_b200 import _lib
+    lib = _lib.load()
+    c1, c2, co = LAYERS[case["layer"]]
+    s["case"], s["grid"] = case, (case["batch"], case["d"], case["h"], case["w"])
+    for key, tr in (("fw", 0), ("bw", 1)):
+        s[key] = torch.empty(27 * co * (c1 + c2), dtype=torch.bfloat16, device="cuda")
+        _lib.check(lib.trtt_b200_conv3_pack(_ptr(s["w"]), co, c1 + c2, tr, _ptr(s[key]), _stream()), "conv3_pack")
+    s["y"] = torch.zeros_like(s["gy"])
+    if case["train"]:
+        s["dx1"], s["dx2"] = torch.zeros_like(s["x1"]), torch.zeros_like(s["x2"]) if c2 else None
+        s["dw"], s["db"] = torch.zeros_like(s["w"]), torch.zeros_like(s["b"])
+        s["nscratch"] = lib.trtt_b200_conv3_wgrad_scratch(co, c1 + c2, *s["grid"])
+        s["scratch"] = torch.empty(s["nscratch"] // 4 + 1, device="cuda")
+    return s
+
+
+def _run_conv(s):
+    from yoricktrtt_b200 import _lib
+    lib = _lib.load()
+    c1, c2, co = LAYERS[s["case"]["layer"]]
+    _lib.check(lib.trtt_b200_conv3_forward(
+        _ptr(s["x1"]), c1, _ptr(s["x2"]), c2, _ptr(s["fw"]), co, _ptr(s["b"]), 0, SLOPE, _ptr(s["y"]), None, 0, 0,
+        None, *s["grid"], _stream()), "conv3_forward")
+    if not s["case"]["train"]:
+        return s["y"]
+    _lib.check(lib.trtt_b200_conv3_forward(
+        _ptr(s["gy"]), co, None, 0, _ptr(s["bw"]), c1 + c2, None, 3, 1.0, _ptr(s["dx1"]), _ptr(s["dx2"]), c1, 0,
+        None, *s["grid"], _stream()), "conv3 input gradient")
+    _lib.check(lib.trtt_b200_conv3_wgrad(
+        _ptr(s["gy"]), co, _ptr(s["x1"]), c1, _ptr(s["x2"]), c2, _ptr(s["dw"]), _ptr(s["db"]), _ptr(s["scratch"]),
+        s["nscratch"], *s["grid"], _stream()), "conv3_wgrad")
+    return {k: s[k] for k in ("y", "dx1", "dx2", "dw", "db") if s[k] is not None}
+
+
 def prepare(case, seed):
     inp = _inputs(case, seed)
     s = {"case": case}
-    if case["kind"] == "unet":
-        from yoricktrtt_b200.unet import UNet3D
-        s["net"] = UNet3D.load(WEIGHTS, lr=1e-3)
-        s["x"], s["target"] = inp["x"], inp["target"]
-        return s
+    if case["kind"] == "conv":
+        return _prepare_conv(case, inp)
     pr = s["pr"] = _projector(case, inp["theta"])
     s["y"] = inp["y"]
     if case["kind"] == "gates4d":
@@ -293,12 +350,8 @@ def prepare(case, seed):
 def run(state):
     case = state["case"]
     kind = case["kind"]
-    if kind == "unet":
-        net = state["net"]
-        if not case["train"]:
-            return net.forward(state["x"])
-        loss = net.train_step(state["x"], state["target"])
-        return {"loss": loss.float(), "params": net.params}
+    if kind == "conv":
+        return _run_conv(state)
     pr, vol, y = state["pr"], state["vol"], state["y"]
     if kind == "pair3d":
         return {"sino": pr.forward(vol, layout=case["layout"]), "back": pr.backward(y, layout=case["layout"])}
@@ -318,20 +371,16 @@ def run(state):
 # ---------------------------------------------------------------------------
 # what a pass cannot do without
 # ---------------------------------------------------------------------------
-LAYERS = [("e1a", 1, 16, 0), ("e1b", 16, 16, 0), ("e2a", 16, 32, 1), ("e2b", 32, 32, 1), ("e3a", 32, 64, 2),
-          ("e3b", 64, 64, 2), ("d2a", 96, 32, 1), ("d2b", 32, 32, 1), ("d1a", 48, 16, 0), ("d1b", 16, 16, 0),
-          ("head", 16, 1, 0)]  # name, true input and output channels, level
-
-
 def work(case):
-    if case["kind"] == "unet":
+    if case["kind"] == "conv":
+        c1, c2, co = LAYERS[case["layer"]]
         vox = case["batch"] * case["d"] * case["h"] * case["w"]
-        params = sum(27 * ci * co + co for _, ci, co, _ in LAYERS)
-        flops = sum(2 * 27 * ci * co * vox / 8 ** lv for _, ci, co, lv in LAYERS)
-        if case["train"]:  # forward, input gradient (not of the input), weight gradient
-            first = 2 * 27 * 16 * vox
-            return {"bytes": 4 * (2 * vox + 6 * params), "flops": 3 * flops - first}
-        return {"bytes": 4 * (2 * vox + params), "flops": flops}
+        ci, wts = c1 + c2, 27 * (c1 + c2) * co
+        flops = 2 * vox * wts
+        if not case["train"]:
+            return {"bytes": 2 * (vox * (ci + co) + wts), "flops": flops}
+        # x, gy in, y, dx out; weights in, their gradients out
+        return {"bytes": 2 * vox * (2 * ci + 2 * co) + 8 * wts, "flops": 3 * flops}
     # footprints of a cubic B-spline: 4 voxels wide, about 4 s magn / d + 1
     # cells; per voxel and view one cell edge costs about 10 operations and a
     # cell 2 more, per column, view and detector cell of its profile 2 per row
@@ -553,49 +602,35 @@ def _tv(x, mu, eps):
     return float(f), torch.autograd.grad(f, x)[0]
 
 
-def _exact_unet(case, inp):
+def _exact_conv(case, inp):
     import torch.nn.functional as F
-    sd = np.load(WEIGHTS)
-    scale = float(sd["scale"])
-    grad = case["train"]
-    P = {k: torch.tensor(sd[k], device="cuda", dtype=torch.float64).requires_grad_(grad)
-         for k in sd.files if k != "scale"}
 
-    def conv(name, t, act=True):
-        w = P[name + ".w"]
-        y = F.conv3d(t, w.permute(0, 2, 1).reshape(w.shape[0], w.shape[2], 3, 3, 3), P[name + ".b"], padding=1)
-        return F.leaky_relu(y, SLOPE) if act else y
+    def dense(a):  # padded channels-last -> (batch, c, d, h, w)
+        return a[:, 1:-1, 1:-1, 1:-1].permute(0, 4, 1, 2, 3).double().contiguous()
 
-    def up(t):
-        return F.interpolate(t, scale_factor=2, mode="nearest")
+    def padded(a):
+        return F.pad(a.permute(0, 2, 3, 4, 1), (0, 0, 1, 1, 1, 1, 1, 1)).contiguous()
 
-    with torch.set_grad_enabled(grad):
-        x = inp["x"].double() * scale
-        xin = torch.zeros((x.shape[0], 16) + tuple(x.shape[1:]), device="cuda", dtype=torch.float64)
-        xin[:, 0] = x
-        e1 = conv("e1b", conv("e1a", xin))
-        e2 = conv("e2b", conv("e2a", F.avg_pool3d(e1, 2)))
-        e3 = conv("e3b", conv("e3a", F.avg_pool3d(e2, 2)))
-        d2 = conv("d2b", conv("d2a", torch.cat([up(e3), e2], 1)))
-        d1 = conv("d1b", conv("d1a", torch.cat([up(d2), e1], 1)))
-        out = x + conv("head", d1, act=False)[:, 0]
-        if not grad:
-            return out / scale
-        loss = ((out - scale * inp["target"].double()) ** 2).mean()
-        loss.backward()
-    params = {}
-    for k, p in P.items():  # first Adam step from zero moments
-        g = p.grad
-        layer, part = k.split(".")
-        params.setdefault(layer, {})[part] = (p - 1e-3 * g / (g.abs() + 1e-8)).detach()
-    return {"loss": loss.detach().reshape(1), "params": params}
+    c1, c2, co = LAYERS[case["layer"]]
+    x = torch.cat([dense(inp[k]) for k in ("x1", "x2") if inp[k] is not None], 1).requires_grad_(case["train"])
+    w = inp["w"].double().requires_grad_(case["train"])
+    b = inp["b"].double().requires_grad_(case["train"])
+    y = F.conv3d(x, w.permute(0, 2, 1).reshape(co, c1 + c2, 3, 3, 3), b, padding=1)
+    out = padded(F.leaky_relu(y.detach(), SLOPE))
+    if not case["train"]:
+        return out
+    y.backward(dense(inp["gy"]))  # the gradient given is that of the layer's linear output
+    d = {"y": out, "dx1": padded(x.grad[:, :c1]), "dw": w.grad, "db": b.grad}
+    if c2:
+        d["dx2"] = padded(x.grad[:, c1:])
+    return d
 
 
 def exact(case, seed):
     inp = _inputs(case, seed)
     kind = case["kind"]
-    if kind == "unet":
-        return _exact_unet(case, inp)
+    if kind == "conv":
+        return _exact_conv(case, inp)
     two_d = kind == "pair2d" or (kind == "objective" and case["nz"] == 0)
     E = _Exact2D(case) if two_d else _Exact3D(case)
     vol, theta = inp["vol"].double(), inp["theta"]
