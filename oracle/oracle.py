@@ -72,7 +72,7 @@ def build(ref: bool = False) -> None:
     """Build the oracle (and, if asked and the reference tree exists, the
     compiled reference) with oracle/Makefile."""
     subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
-    if ref and os.path.isdir(REFROOT):
+    if ref and os.path.exists(os.path.join(REFROOT, "plugin", "trtt_common.c")):
         subprocess.run(["make", "-s", "-C", HERE, "ref", f"REFROOT={REFROOT}"], check=True)
 
 
