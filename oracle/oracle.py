@@ -232,4 +232,4 @@ def get(kind: str = "port") -> Oracle:
 
 
 def ref_available() -> bool:
-    return os.path.exists(REF_SO) or os.path.isdir(REFROOT)
+    return os.path.exists(REF_SO) or os.path.exists(os.path.join(REFROOT, "plugin", "trtt_common.c"))
