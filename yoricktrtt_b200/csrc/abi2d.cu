@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "kernels2d.h"
+#include "proj2d_orbit.cuh"
 #include "runtime.h"
 #include "trtt_b200.h"
 
@@ -124,6 +125,52 @@ int check_flag(DropIn &D, const char *what)
   return 0;
 }
 
+Orbit2DLaunch orbit_launch(const Orbit2DScan &scan, const Orbit2D *groups_dev, const Params2D &P,
+                           const View2D *views, const float *in, float *out)
+{
+  Orbit2DLaunch L;
+  std::memset(&L, 0, sizeof(L));
+  L.P = P;
+  L.views = views;
+  L.groups = groups_dev;
+  L.ngroups = (int)scan.groups.size();
+  L.model = scan.model;
+  L.cls = scan.cls;
+  L.line = scan.line;
+  L.in = in;
+  L.out = out;
+  return L;
+}
+
+// Direct (job 0) or transpose of a scan on the drop-in state's stream, by the
+// group kernels when the scan takes that path (`ok`; its records go to
+// D.grp).  *done: launched.
+cudaError_t dropin_orbit(DropIn &D, const Orbit2DScan &scan, bool ok, const Params2D &P, const View2D *views,
+                         const float *in, float *out, int job, bool *done)
+{
+  *done = false;
+  if (!ok) return cudaSuccess;
+  const size_t bytes = sizeof(Orbit2D) * scan.groups.size();
+  cudaError_t e = D.grp.ensure(bytes);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(D.grp.p, scan.groups.data(), bytes, cudaMemcpyHostToDevice, D.stream);
+  if (e != cudaSuccess) return e;
+  const Orbit2DLaunch L = orbit_launch(scan, D.grp.as<Orbit2D>(), P, views, in, out);
+  *done = true;
+  return job == 0 ? launch_fwd2d_orbit(L, D.stream) : launch_back2d_orbit(L, D.stream);
+}
+
+// Sizes of a Long-Fessler scan as the group kernels take them.
+Params2D lf_params2d(const LFView &g)
+{
+  Params2D P;
+  std::memset(&P, 0, sizeof(P));
+  P.nx = g.n1;
+  P.ny = g.n2;
+  P.nv = g.nd;
+  P.hs0 = g.size;
+  return P;
+}
+
 // out += H in (job 0) or H^T in (job != 0) on host arrays, one or more views.
 int host2d(int fan, double *out, const double *in, long nx, long ny, double s_scl, int s_deg,
            const double *cum, long size, double step, const double *coord, long nv,
@@ -163,7 +210,13 @@ int host2d(int fan, double *out, const double *in, long nx, long ny, double s_sc
   TRTT_CK(D.det32.ensure(sizeof(float) * nout));
   TRTT_CK(f64_to_f32(D.in64.as<double>(), D.vol32.as<float>(), nin, st));
   TRTT_CK(cudaMemsetAsync(D.det32.p, 0, sizeof(float) * nout, st));
-  if (job == 0)
+  Orbit2DScan scan;
+  bool done = false;
+  TRTT_CK(dropin_orbit(D, scan, orbit2d_bspline(P, hv.data(), nviews, xos, xsd, scan), P, D.geom.as<View2D>(),
+                       D.vol32.as<float>(), D.det32.as<float>(), job, &done));
+  if (done)
+    ;
+  else if (job == 0)
     TRTT_CK(launch_fwd2d(P, D.geom.as<View2D>(), (int)nviews, D.vol32.as<float>(),
                          D.det32.as<float>(), D.err.as<int>(), st));
   else
@@ -257,7 +310,13 @@ void host_lf(const void *pv, double beta, double offset, const double *src, doub
   LF_CK(D.det32.ensure(sizeof(float) * nout));
   LF_CK(f64_to_f32(D.in64.as<double>(), D.vol32.as<float>(), nin, st));
   LF_CK(cudaMemsetAsync(D.det32.p, 0, sizeof(float) * nout, st));
-  if (direct)
+  Orbit2DScan scan;
+  bool done = false;
+  LF_CK(dropin_orbit(D, scan, orbit2d_lf(&g, 1, line, scan), lf_params2d(g), nullptr, D.vol32.as<float>(),
+                     D.det32.as<float>(), direct ? 0 : 1, &done));
+  if (done)
+    ;
+  else if (direct)
     LF_CK(launch_lf_fwd(D.geom.as<LFView>(), 1, (int)nd, line, D.vol32.as<float>(), D.det32.as<float>(), st));
   else
     LF_CK(launch_lf_back(D.geom.as<LFView>(), 1, (int)npix, line, D.vol32.as<float>(), D.det32.as<float>(), st));
@@ -607,7 +666,26 @@ struct trtt_b200_plan2d {
   long nviews = 0, npix = 0, ndet = 0;
   Params2D P;
   DevBuf views, cum, err;
+  Orbit2DScan orbit;   // view groups; empty: the per-view kernels
+  DevBuf groups;
 };
+
+namespace {
+
+// The plan's groups on the device (none: the scan keeps the per-view kernels).
+cudaError_t upload_orbit(trtt_b200_plan2d *pl, bool ok)
+{
+  if (!ok) {
+    pl->orbit.groups.clear();
+    return cudaSuccess;
+  }
+  const size_t bytes = sizeof(Orbit2D) * pl->orbit.groups.size();
+  cudaError_t e = pl->groups.ensure(bytes);
+  if (e == cudaSuccess) e = cudaMemcpy(pl->groups.p, pl->orbit.groups.data(), bytes, cudaMemcpyHostToDevice);
+  return e;
+}
+
+}  // namespace
 
 extern "C" int trtt_b200_plan2d_create(trtt_b200_plan2d **plan, int geometry, long nx, long ny,
                                        double s_scl, int s_deg, const double *cum_footprint,
@@ -645,6 +723,7 @@ extern "C" int trtt_b200_plan2d_create(trtt_b200_plan2d **plan, int geometry, lo
     e = cudaMemcpy(pl->views.p, hv.data(), sizeof(View2D) * nviews, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = pl->err.ensure(sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(pl->err.p, 0, sizeof(int));
+  if (e == cudaSuccess) e = upload_orbit(pl, orbit2d_bspline(pl->P, hv.data(), nviews, xos, xsd, pl->orbit));
   if (e != cudaSuccess) {
     delete pl;
     return fail_cuda(e, "plan2d_create");
@@ -678,10 +757,12 @@ extern "C" int trtt_b200_plan2d_create_lf(trtt_b200_plan2d **plan, const void *p
     e = cudaMemcpy(pl->views.p, hv.data(), sizeof(LFView) * nviews, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = pl->err.ensure(sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(pl->err.p, 0, sizeof(int));
+  if (e == cudaSuccess) e = upload_orbit(pl, orbit2d_lf(hv.data(), nviews, pl->line, pl->orbit));
   if (e != cudaSuccess) {
     delete pl;
     return fail_cuda(e, "plan2d_create_lf");
   }
+  pl->P = lf_params2d(hv[0]);
   pl->nviews = nviews;
   pl->npix = p->objectDimension1 * p->objectDimension2;
   pl->ndet = p->detectorDimension;
@@ -695,7 +776,9 @@ extern "C" int trtt_b200_plan2d_forward(trtt_b200_plan2d *pl, const float *img, 
   clear_error();
   if (!pl || !img || !sino) return fail("plan2d_forward: null argument");
   cudaStream_t st = (cudaStream_t)stream;
-  if (pl->lf)
+  if (!pl->orbit.groups.empty())
+    TRTT_CK(launch_fwd2d_orbit(orbit_launch(pl->orbit, pl->groups.as<Orbit2D>(), pl->P, pl->views.as<View2D>(), img, sino), st));
+  else if (pl->lf)
     TRTT_CK(launch_lf_fwd(pl->views.as<LFView>(), (int)pl->nviews, (int)pl->ndet, pl->line, img, sino, st));
   else
     TRTT_CK(launch_fwd2d(pl->P, pl->views.as<View2D>(), (int)pl->nviews, img, sino, pl->err.as<int>(), st));
@@ -709,7 +792,9 @@ extern "C" int trtt_b200_plan2d_backward(trtt_b200_plan2d *pl, const float *sino
   clear_error();
   if (!pl || !img || !sino) return fail("plan2d_backward: null argument");
   cudaStream_t st = (cudaStream_t)stream;
-  if (pl->lf)
+  if (!pl->orbit.groups.empty())
+    TRTT_CK(launch_back2d_orbit(orbit_launch(pl->orbit, pl->groups.as<Orbit2D>(), pl->P, pl->views.as<View2D>(), sino, img), st));
+  else if (pl->lf)
     TRTT_CK(launch_lf_back(pl->views.as<LFView>(), (int)pl->nviews, (int)pl->npix, pl->line, sino, img, st));
   else
     TRTT_CK(launch_back2d(pl->P, pl->views.as<View2D>(), (int)pl->nviews, sino, img, pl->err.as<int>(), st));
@@ -736,6 +821,7 @@ extern "C" int trtt_b200_plan2d_destroy(trtt_b200_plan2d *pl)
   pl->views.release();
   pl->cum.release();
   pl->err.release();
+  pl->groups.release();
   delete pl;
   return 0;
 }
