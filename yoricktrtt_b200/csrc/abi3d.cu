@@ -33,6 +33,8 @@ struct trtt_b200_plan3d {
   int pull = 0;  // 1: atomic-free band kernel (closed-form model, nu <= 512)
   int tc = 0;    // 1: tensor-core band kernel (closed-form model)
   int cols = 1;  // 2: column-pair band kernel (closed-form model)
+  bool tiles_set = false;  // a band kernel was asked for (set_tiles)
+  SweepBounds sweep = {0, 0, 0, 0, 0};  // direct projection by sweeps (rows 0: does not apply)
   bool factorized = true;
   DevBuf views, cum, gate_ptr, entries, pairs, scratch, err;
   std::vector<View3D> hviews;
@@ -42,10 +44,12 @@ struct trtt_b200_plan3d {
   bool grouped = false;   // groups were found (some group has 2 or 4 views)
   int ngroups[3] = {0, 0, 0};
   DevBuf groups[3];
+  bool group_set = false;       // a shape of the direct group kernel was asked for
   int gband[3] = {64, 32, 32};  // direct: band rows per group size
   int gutile4 = 0, gminb4 = 1;  // direct, quads: cells per u tile (0: up to 256), CTAs per SM
   long back_chunk_bytes = 32L << 20;  // transpose: detector bytes per launch
   // persistent weighted least-squares launch
+  bool wls_set = false;    // a shape of the persistent launch was asked for
   int wls_rows = 32, wls_ctas = 1, wls_extra = 0;
   long long wls_wait_ns = 2000000000LL;
   DevBuf resid, wls_parts, wls_queue;
@@ -60,6 +64,46 @@ static bool use_groups(const trtt_b200_plan3d *pl, long view0, long nview)
   return pl->sym && pl->grouped && pl->factorized && pl->P.model == MODEL_CUBIC && pl->nt == 1 &&
          !pl->pull && !pl->tc && pl->cols == 1 && view0 == 0 && nview == pl->nviews &&
          pl->nviews <= 65535;
+}
+
+// Per-view launches of views [view0, view0 + nview) (column layout).
+static Fwd3DLaunch fwd_launch(const trtt_b200_plan3d *pl, const float *vol, float *sino, long view0, long nview)
+{
+  Fwd3DLaunch L;
+  L.P = pl->P;
+  L.views = pl->views.as<View3D>() + view0;
+  L.nviews = (int)nview;
+  L.vol = vol;
+  L.gate_stride = (long)pl->P.nx * pl->P.ny * pl->P.nz;
+  L.sino = sino;
+  L.sino_view_stride = (long)pl->P.nu * pl->P.nv;
+  L.band_rows = pl->factorized ? pl->band_rows : 0;
+  L.warps = pl->warps;
+  L.pull = pl->pull;
+  L.tc = pl->tc;
+  L.cols = pl->cols;
+  L.err = pl->err.as<int>();
+  return L;
+}
+
+static Back3DLaunch back_launch(const trtt_b200_plan3d *pl, const float *sino, float *vol, long view0, long nview)
+{
+  Back3DLaunch L;
+  L.P = pl->P;
+  L.views = pl->views.as<View3D>();
+  L.gate_ptr = pl->gate_ptr.as<int>();
+  L.entries = pl->entries.as<GateEntry>();
+  L.ngates = pl->nt;
+  L.view_lo = (int)view0;
+  L.view_hi = (int)(view0 + nview);
+  L.sino = sino;
+  L.sino_view_stride = (long)pl->P.nu * pl->P.nv;
+  L.vol = vol;
+  L.gate_stride = (long)pl->P.nx * pl->P.ny * pl->P.nz;
+  L.factorized = pl->factorized ? 1 : 0;
+  L.pairs = pl->nt > 1 ? pl->pairs.as<GatePair>() : nullptr;
+  L.err = pl->err.as<int>();
+  return L;
 }
 
 static int upload_gates(trtt_b200_plan3d *pl, const std::vector<std::vector<GateEntry>> &lists)
@@ -135,6 +179,7 @@ extern "C" int trtt_b200_plan3d_create(trtt_b200_plan3d **plan, int geometry,
     if (!pl->hviews[v].factorized) pl->factorized = false;
   }
   choose_band(pl->P.nu, pl->P.nv, pl->band_rows, pl->warps);
+  if (pl->factorized && !cum_footprint) pl->sweep = sweep_bounds(pl->P, pl->hviews.data(), nviews);
   if (pl->factorized && !cum_footprint) {
     std::vector<int> lists[3];
     find_view_groups(nx, ny, nviews, xos, xsd, lists);
@@ -210,6 +255,7 @@ extern "C" int trtt_b200_plan3d_set_tiles(trtt_b200_plan3d *pl, int band_rows, i
 {
   clear_error();
   if (!pl) return fail("plan3d_set_tiles: null plan");
+  pl->tiles_set = !(band_rows == 0 && warps == 0);
   if (band_rows == 0 && warps == 0) {  // defaults
     pl->pull = 0;
     pl->tc = 0;
@@ -293,7 +339,10 @@ extern "C" int trtt_b200_plan3d_set_group_tiles(trtt_b200_plan3d *pl, int band_r
       return fail("plan3d_set_group_tiles: band does not fit in shared memory");
   }
   for (int q = 0; q < 3; ++q)
-    if (req[q]) pl->gband[q] = req[q];
+    if (req[q]) {
+      pl->gband[q] = req[q];
+      pl->group_set = true;
+    }
   if (back_chunk_bytes < 0) return fail("plan3d_set_group_tiles: negative chunk size");
   if (back_chunk_bytes) pl->back_chunk_bytes = back_chunk_bytes;
   return 0;
@@ -316,6 +365,7 @@ extern "C" int trtt_b200_plan3d_set_persistent(trtt_b200_plan3d *pl, int band_ro
     pl->wls_rows = band_rows;
   }
   if (ctas_per_sm) pl->wls_ctas = ctas_per_sm;
+  if (band_rows || ctas_per_sm) pl->wls_set = true;
   if (wait_seconds > 0.0) pl->wls_wait_ns = (long long)(wait_seconds * 1e9);
   pl->wls_extra = extra_wait;
   return 0;
@@ -330,6 +380,24 @@ extern "C" int trtt_b200_plan3d_wls_grad(trtt_b200_plan3d *pl, const float *vol,
     return fail("plan3d_wls_grad: needs the closed-form model and column-factorised views");
   cudaStream_t st = (cudaStream_t)stream;
   const Params3D &P = pl->P;
+  if (!pl->wls_set && pl->wls_extra == 0 && pl->band_rows > 0 && pl->nviews <= 65535) {
+    // direct projection, residual with its cost, transpose: three launches, each
+    // at its own shape.  10 gates of 128 x 128 x 64, 347 views on 256^2: 24.4 ms;
+    // the persistent launch 26.0 at its best shape and 28.5-33 at its default
+    // one.  The direct projection is the band kernel, whose FP32 sums are the
+    // persistent launch's: the FP64 cost shows their rounding (8e-8 below the
+    // exact value), and callers compare costs to 1e-9.
+    const long npix = (long)P.nu * P.nv;
+    TRTT_CK(pl->resid.ensure(sizeof(float) * (size_t)pl->nviews * npix));
+    float *resid = pl->resid.as<float>();
+    TRTT_CK(cudaMemsetAsync(resid, 0, sizeof(float) * (size_t)pl->nviews * npix, st));
+    TRTT_CK(cudaMemsetAsync(cost, 0, sizeof(double), st));
+    TRTT_CK(launch_fwd3d(fwd_launch(pl, vol, resid, 0, pl->nviews), st));
+    TRTT_CK(launch_wls_residual(resid, y, w, pl->nviews * npix, cost, st));
+    TRTT_CK(launch_back3d(back_launch(pl, resid, grad, 0, pl->nviews), st));
+    count_launch(3);
+    return 0;
+  }
   int dev = 0, sms = 0, coop = 0;
   TRTT_CK(cudaGetDevice(&dev));
   TRTT_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -384,6 +452,7 @@ extern "C" int trtt_b200_plan3d_set_group_shape(trtt_b200_plan3d *pl, int band_r
   const size_t smem = group_fwd_smem(4, rows, ut, group_fwd_warps(4, rows, ut, cpsm));
   if (smem > (cpsm == 2 ? 113u : 227u) * 1024u)
     return fail("plan3d_set_group_shape: the quad band does not fit in shared memory at that occupancy");
+  if (band_rows4 || utile4 || ctas_per_sm4) pl->group_set = true;
   if (band_rows4) pl->gband[2] = band_rows4;
   pl->gutile4 = utile4;
   if (ctas_per_sm4) pl->gminb4 = ctas_per_sm4;
@@ -439,6 +508,22 @@ static int plan_run(trtt_b200_plan3d *pl, const float *src, float *dst, long vie
     for (int q = 2; q >= 0; --q) {
       if (!pl->ngroups[q]) continue;
       const int G = group_size_of(q);
+      if (pl->sweep.rows > 0 && pl->sym == 2 && !pl->group_set) {
+        SweepLaunch S;
+        S.P = P;
+        S.views = pl->views.as<View3D>();
+        S.groups = pl->groups[q].as<int>();
+        S.count = pl->ngroups[q];
+        S.b = pl->sweep;
+        S.vol = volc;
+        S.gate_stride = nvox;
+        S.sino = dst;
+        S.sino_view_stride = npix;
+        S.err = pl->err.as<int>();
+        TRTT_CK(launch_fwd3d_sweep(S, G, st));
+        count_launch();
+        continue;
+      }
       GroupFwdLaunch L;
       L.P = P;
       L.views = pl->views.as<View3D>();
@@ -488,39 +573,12 @@ static int plan_run(trtt_b200_plan3d *pl, const float *src, float *dst, long vie
       count_launch();
     }
   } else if (forward) {
-    Fwd3DLaunch L;
-    L.P = P;
-    L.views = pl->views.as<View3D>() + view0;
-    L.nviews = (int)nview;
-    L.vol = volc;
-    L.gate_stride = nvox;
-    L.sino = dst;
-    L.sino_view_stride = npix;
-    L.band_rows = pl->factorized ? pl->band_rows : 0;
-    L.warps = pl->warps;
-    L.pull = pl->pull;
-    L.tc = pl->tc;
-    L.cols = pl->cols;
-    L.err = pl->err.as<int>();
+    Fwd3DLaunch L = fwd_launch(pl, volc, dst, view0, nview);
+    if (!pl->tiles_set && pl->cols == 1) L.sweep = pl->sweep;
     TRTT_CK(launch_fwd3d(L, st));
     count_launch();
   } else {
-    Back3DLaunch L;
-    L.P = P;
-    L.views = pl->views.as<View3D>();
-    L.gate_ptr = pl->gate_ptr.as<int>();
-    L.entries = pl->entries.as<GateEntry>();
-    L.ngates = pl->nt;
-    L.view_lo = (int)view0;
-    L.view_hi = (int)(view0 + nview);
-    L.sino = src;
-    L.sino_view_stride = npix;
-    L.vol = volo;
-    L.gate_stride = nvox;
-    L.factorized = pl->factorized ? 1 : 0;
-    L.pairs = pl->nt > 1 ? pl->pairs.as<GatePair>() : nullptr;
-    L.err = pl->err.as<int>();
-    TRTT_CK(launch_back3d(L, st));
+    TRTT_CK(launch_back3d(back_launch(pl, src, volo, view0, nview), st));
     count_launch();
     if (layout == TRTT_B200_LAYOUT_XYZ) {
       TRTT_CK(col_f32_add_to_xyz_f32(volo, dst, P.nx, P.ny, P.nz, pl->nt, st));
@@ -641,7 +699,8 @@ void member_runs(const std::vector<int> &list, int G, long g0, long g1,
 // stream, ordered after ev[0].
 int host3d_grouped(DropIn &D, const Params3D &P, double *out, const double *in,
                    const std::vector<int> (&lists)[3], long nviews, int job,
-                   const std::function<cudaError_t(cudaStream_t)> &out_to_device, bool in_early)
+                   const std::function<cudaError_t(cudaStream_t)> &out_to_device, bool in_early,
+               const SweepBounds &sweep)
 {
   cudaStream_t st = D.stream, cp = D.copy, ks2 = D.stream2;
   const long nx = P.nx, ny = P.ny, nz = P.nz, nu = P.nu, nv = P.nv;
@@ -700,7 +759,22 @@ int host3d_grouped(DropIn &D, const Params3D &P, double *out, const double *in,
         cudaStream_t ks = (unit & 1) ? ks2 : st;
         L.groups = D.grp.as<int>() + offs[q] + 4 * cb[c];
         L.ngroups = (int)(cb[c + 1] - cb[c]);
-        TRTT_CK(launch_fwd3d_group(L, G, ks));
+        if (sweep.rows > 0) {
+          SweepLaunch S;
+          S.P = P;
+          S.views = L.views;
+          S.groups = L.groups;
+          S.count = L.ngroups;
+          S.b = sweep;
+          S.vol = L.vol;
+          S.gate_stride = nvox;
+          S.sino = L.sino;
+          S.sino_view_stride = nview_px;
+          S.err = L.err;
+          TRTT_CK(launch_fwd3d_sweep(S, G, ks));
+        } else {
+          TRTT_CK(launch_fwd3d_group(L, G, ks));
+        }
         TRTT_CK(cudaEventRecord(D.ev[ev], ks));
         TRTT_CK(cudaStreamWaitEvent(cp, D.ev[ev], 0));
         ++ev;
@@ -846,10 +920,12 @@ int host3d(int geom, double *out, const double *in, long nx, long ny, long nz,
       std::fprintf(stderr, "trtt_b200: a voxel lies in the source plane (wk == 0); out left unchanged\n");
       return fail("a voxel lies in the source plane (wk == 0)");
     }
-    return host3d_grouped(D, P, out, in, glists, nviews, job, out_to_device, in_early);
+    return host3d_grouped(D, P, out, in, glists, nviews, job, out_to_device, in_early,
+                          sweep_bounds(P, hv.data(), nviews));
   }
   if (grouped) {
-    const int r = host3d_grouped(D, P, out, in, glists, nviews, job, out_to_device, in_early);
+    const int r = host3d_grouped(D, P, out, in, glists, nviews, job, out_to_device, in_early,
+                          sweep_bounds(P, hv.data(), nviews));
     if (r < 0) return r;
   } else if (job == 0 && fact) {
     // Column-factorised views: the only failure (a voxel in the source
@@ -883,6 +959,7 @@ int host3d(int geom, double *out, const double *in, long nx, long ny, long nz,
     choose_band((int)nu, (int)nv, rows, warps);
     L.band_rows = rows;
     L.warps = warps;
+    if (P.model == MODEL_CUBIC) L.sweep = sweep_bounds(P, hv.data(), nviews);
     L.err = D.err.as<int>();
     const long bands = (nv + rows - 1) / rows;
     const std::vector<long> cb = fwd_chunks(nviews, (nviews + 5) / 6, std::max<long>(1, 2L * D.sms / bands),

@@ -212,6 +212,61 @@ inline void choose_band(int nu, int nv, int &band_rows, int &warps)
   band_rows = rows >= 2 ? (int)rows : 0;
 }
 
+// Bounds for the sweep kernel over the factorised views of a closed-form plan:
+// the detector rows of one voxel column's v footprint, and the part of the
+// detector that any footprint can reach (a volume's shadow seldom fills the
+// detector; the tiles cover no more than it).  rows = 0 where the kernel does
+// not apply: a footprint that is not the cubic's 4 voxels wide (its walk
+// starts at a zero of the primitive), a source within the volume.
+inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nviews)
+{
+  SweepBounds b = {0, 0, 0, 0, 0};
+  if (P.hs0 != 2.0) return b;
+  double hsv = 0.0, hsu = 0.0, u0 = HUGE_VAL, u1 = -HUGE_VAL, v0 = HUGE_VAL, v1 = -HUGE_VAL;
+  for (long n = 0; n < nviews; ++n) {
+    const View3D &V = views[n];
+    double wmin = HUGE_VAL, wmax = -HUGE_VAL, dv2 = 0.0, du2 = 0.0;
+    for (int c = 0; c < 8; ++c) {
+      const double i = (c & 1) ? P.nx - 1 : 0, j = (c & 2) ? P.ny - 1 : 0, k = (c & 4) ? P.nz - 1 : 0;
+      double u, v;
+      if (P.geom == GEOM_CONE) {
+        const double w = V.o1 * i + V.o2 * j + V.o4, q = V.a4m / (V.d_x * i + V.d_y * j + V.d_c);
+        v = q * (V.nv_x * i + V.nv_y * j + V.nv_c) + V.b3;
+        u = q * (V.nu_x * i + V.nu_y * j + V.nu_z * k + V.nu_c) + V.c3;
+        wmin = std::fmin(wmin, w);
+        wmax = std::fmax(wmax, w);
+        const double va = (v - V.a8) * P.v_scl, ua = (u - V.a12) * P.u_scl;
+        dv2 = std::fmax(dv2, va * va / V.a4sqr);
+        du2 = std::fmax(du2, ua * ua / V.a4sqr);
+      } else {
+        v = V.v_x * i + V.v_y * j + V.v_c;
+        u = V.u_x * i + V.u_y * j + V.u_z * k + V.u_c;
+      }
+      u0 = std::fmin(u0, u);
+      u1 = std::fmax(u1, u);
+      v0 = std::fmin(v0, v);
+      v1 = std::fmax(v1, v);
+    }
+    if (P.geom == GEOM_CONE) {
+      if (!(wmin * wmax > 0.0)) return b;
+      // nearest corner: largest magnification; outermost: largest obliquity
+      const double magn = std::fabs(V.a4m) / std::fmin(std::fabs(wmin), std::fabs(wmax));
+      hsv = std::fmax(hsv, P.hs0 * P.h_v0 * magn * std::sqrt(1.0 + dv2));
+      hsu = std::fmax(hsu, P.hs0 * P.h_u0 * magn * std::sqrt(1.0 + du2));
+    } else {
+      hsv = std::fmax(hsv, V.p_hs_v);
+      hsu = std::fmax(hsu, V.p_hs_u);
+    }
+  }
+  if (!(hsv > 0.0 && hsv < 1e4 && hsu < 1e4 && u0 > -1e8 && u1 < 1e8 && v0 > -1e8 && v1 < 1e8)) return b;
+  b.rows = (int)std::floor(2.0 * hsv * 1.0001) + 2;
+  b.u0 = (int)std::fmin(std::fmax(std::floor(u0 - hsu * 1.0001) - 1.0, 0.0), P.nu);
+  b.u1 = (int)std::fmin(std::fmax(std::ceil(u1 + hsu * 1.0001) + 2.0, 0.0), P.nu);
+  b.v0 = (int)std::fmin(std::fmax(std::floor(v0 - hsv * 1.0001) - 1.0, 0.0), P.nv);
+  b.v1 = (int)std::fmin(std::fmax(std::ceil(v1 + hsv * 1.0001) + 2.0, 0.0), P.nv);
+  return b;
+}
+
 inline int geom_code(int geometry)
 {
   if (geometry == TRTT_B200_PARALLEL_BEAM) return GEOM_PARALLEL;

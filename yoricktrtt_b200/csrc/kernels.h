@@ -28,6 +28,13 @@ struct GatePair {
   float w0, w1;
 };
 
+// Bounds of the sweep kernel (sweep_bounds, host3d.h): detector rows of one
+// voxel column (0: the kernel does not apply), reachable cells [u0, u1) and
+// rows [v0, v1).
+struct SweepBounds {
+  int rows, u0, u1, v0, v1;
+};
+
 struct Fwd3DLaunch {
   Params3D P;
   const View3D *views;   // device, nviews entries
@@ -41,6 +48,7 @@ struct Fwd3DLaunch {
   int pull = 0;          // closed-form model, nu <= 512: atomic-free band kernel
   int cols = 1;          // closed-form model: 2 = column-pair band kernel
   int tc = 0;            // closed-form model: 1 = tensor-core band kernel (rows chosen by it)
+  SweepBounds sweep = {0, 0, 0, 0, 0};  // closed-form model, rows > 0: sweep kernel
   int *err;              // device error flags
 };
 
@@ -80,6 +88,24 @@ struct GroupFwdLaunch {
   int minb = 1;          // groups of 4: 1 CTA per SM (up to 22 warps) or 2 (64 registers per thread)
   int *err;
 };
+
+// Direct projector by sweeps over image lines (proj3d_sweep.cu; closed-form
+// model, column-factorised views) of `count` view groups of `groups` (4 view
+// indices each) or, with groups null, `count` single views; at most 65535.
+struct SweepLaunch {
+  Params3D P;
+  const View3D *views;
+  const int *groups;
+  int count;
+  SweepBounds b;
+  const float *vol;      // column layout [gate][j][i][k]
+  long gate_stride;
+  float *sino;           // [view][nv][nu], accumulated
+  long sino_view_stride;
+  int *err;
+  int band_rows = 0, usplit = 0, utile = 0, split = 0;  // chosen by the launcher
+};
+cudaError_t launch_fwd3d_sweep(const SweepLaunch &L, int G, cudaStream_t st);
 
 // Transpose over orbits of columns under the group's turns, for the groups
 // [g_lo, g_hi) of `groups`.
@@ -138,6 +164,8 @@ __host__ __device__ inline size_t back_gates_row(int nu, int ngates, int kp)
 inline bool band_lock_spread(const Params3D &P) { return P.nz >= 128; }
 int wls_kp(int nz);
 cudaError_t launch_wls_persistent(WlsLaunch L, int sms, cudaStream_t st);
+// hx = W (hx - y) in place, *cost += 1/2 sum W (hx - y)^2 (w may be null)
+cudaError_t launch_wls_residual(float *hx, const float *y, const float *w, long n, double *cost, cudaStream_t st);
 
 size_t group_fwd_smem(int G, int band_rows, int utile, int warps);
 int group_fwd_warps(int G, int band_rows, int utile, int minb);

@@ -102,6 +102,7 @@ extern "C" int trtt_b200_cb3d_cubic_forward_noalloc(const float *vol_columns, fl
   choose_band((int)nu, (int)nv, rows, warps);
   L.band_rows = fact ? rows : 0;
   L.warps = warps;
+  if (fact) L.sweep = sweep_bounds(P, g_host_views, nviews);
   L.err = err_dev;
   TRTT_CK(launch_fwd3d(L, st));
   count_launch();

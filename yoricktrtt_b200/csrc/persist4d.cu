@@ -167,6 +167,29 @@ k_wls_persistent(const WlsLaunch A)
   }
 }
 
+// Residual and cost of the launch-by-launch form.
+__global__ void __launch_bounds__(256) k_wls_residual(float *hx, const float *__restrict__ y,
+                                                      const float *__restrict__ w, long n, double *cost)
+{
+  double c = 0.0;
+  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
+    const float r = hx[t] - __ldg(y + t);
+    const float q = w ? __ldg(w + t) * r : r;
+    hx[t] = q;
+    c += (double)q * (double)r;
+  }
+  __shared__ double red[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(FULLM, c, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int q = 0; q < 8; ++q) s += red[q];
+    atomicAdd(cost, 0.5 * s);
+  }
+}
+
 template <int GEOM, int KP, int MINB>
 cudaError_t launch_wls(WlsLaunch L, int sms, cudaStream_t st)
 {
@@ -185,6 +208,13 @@ cudaError_t launch_wls(WlsLaunch L, int sms, cudaStream_t st)
 }
 
 }  // namespace
+
+cudaError_t launch_wls_residual(float *hx, const float *y, const float *w, long n, double *cost, cudaStream_t st)
+{
+  const long blocks = (n + 1023) / 1024;
+  k_wls_residual<<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, st>>>(hx, y, w, n, cost);
+  return cudaGetLastError();
+}
 
 size_t wls_smem(int nu, int band_rows)
 {

@@ -522,6 +522,20 @@ static cudaError_t back_fast(const Back3DLaunch &L, cudaStream_t st)
 cudaError_t launch_fwd3d_fast(const Fwd3DLaunch &L, cudaStream_t st)
 {
   if (L.tc && L.P.model == MODEL_CUBIC) return launch_fwd3d_tc(L, st);
+  if (L.P.model == MODEL_CUBIC && L.sweep.rows > 0 && L.nviews <= 65535) {
+    SweepLaunch S;
+    S.P = L.P;
+    S.views = L.views;
+    S.groups = nullptr;
+    S.count = L.nviews;
+    S.b = L.sweep;
+    S.vol = L.vol;
+    S.gate_stride = L.gate_stride;
+    S.sino = L.sino;
+    S.sino_view_stride = L.sino_view_stride;
+    S.err = L.err;
+    return launch_fwd3d_sweep(S, 1, st);
+  }
   return L.P.geom == GEOM_CONE ? fwd_fast<GEOM_CONE>(L, st) : fwd_fast<GEOM_PARALLEL>(L, st);
 }
 
