@@ -34,9 +34,10 @@ struct trtt_b200_plan3d {
   int tc = 0;    // 1: tensor-core band kernel (closed-form model)
   int cols = 1;  // 2: column-pair band kernel (closed-form model)
   bool tiles_set = false;  // a band kernel was asked for (set_tiles)
-  SweepBounds sweep = {0, 0, 0, 0, 0};  // direct projection by sweeps (rows 0: does not apply)
+  SweepBounds sweep;       // sweep and gather kernels (rows 0: do not apply)
+  bool gates_set = false;  // weights other than one view, one gate
   bool factorized = true;
-  DevBuf views, cum, gate_ptr, entries, pairs, scratch, err;
+  DevBuf views, cum, gate_ptr, entries, pairs, order, scratch, err;
   std::vector<View3D> hviews;
   // view groups related by turns of the grid (closed-form model, factorised
   // views): index 0 singles, 1 pairs (half turns), 2 quads (quarter turns)
@@ -102,6 +103,12 @@ static Back3DLaunch back_launch(const trtt_b200_plan3d *pl, const float *sino, f
   L.gate_stride = (long)pl->P.nx * pl->P.ny * pl->P.nz;
   L.factorized = pl->factorized ? 1 : 0;
   L.pairs = pl->nt > 1 ? pl->pairs.as<GatePair>() : nullptr;
+  L.sweep = pl->sweep;
+  if (pl->gates_set) {
+    L.order = pl->order.as<int>();
+    L.norder = (int)pl->nviews;
+    L.order_pairs = pl->pairs.as<GatePair>();
+  }
   L.err = pl->err.as<int>();
   return L;
 }
@@ -135,6 +142,15 @@ static int upload_gates(trtt_b200_plan3d *pl, const std::vector<std::vector<Gate
     }
   TRTT_CK(pl->pairs.ensure(sizeof(GatePair) * pairs.size()));
   TRTT_CK(cudaMemcpy(pl->pairs.p, pairs.data(), sizeof(GatePair) * pairs.size(), cudaMemcpyHostToDevice));
+  // the views sorted by their gates, for the transpose that keeps the current
+  // two gates' sums in registers
+  std::vector<int> order(pairs.size());
+  for (size_t v = 0; v < order.size(); ++v) order[v] = (int)v;
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return pairs[a].g0 != pairs[b].g0 ? pairs[a].g0 < pairs[b].g0 : pairs[a].g1 < pairs[b].g1;
+  });
+  TRTT_CK(pl->order.ensure(sizeof(int) * order.size()));
+  TRTT_CK(cudaMemcpy(pl->order.p, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
   return 0;
 }
 
@@ -248,6 +264,7 @@ extern "C" int trtt_b200_plan3d_set_gates(trtt_b200_plan3d *pl, long nt, const d
   TRTT_CK(cudaMemcpy(pl->views.p, pl->hviews.data(), sizeof(View3D) * pl->nviews, cudaMemcpyHostToDevice));
   pl->nt = (int)nt;
   pl->P.nt = (int)nt;
+  pl->gates_set = true;
   return upload_gates(pl, lists);
 }
 
@@ -622,6 +639,7 @@ extern "C" int trtt_b200_plan3d_destroy(trtt_b200_plan3d *pl)
   pl->gate_ptr.release();
   pl->entries.release();
   pl->pairs.release();
+  pl->order.release();
   for (auto &gb : pl->groups) gb.release();
   pl->resid.release();
   pl->wls_parts.release();
@@ -1032,6 +1050,7 @@ int host3d(int geom, double *out, const double *in, long nx, long ny, long nz,
     L.vol = D.vol32.as<float>();
     L.gate_stride = nvox;
     L.factorized = fact ? 1 : 0;
+    if (fact && !cum) L.sweep = sweep_bounds(P, hv.data(), nviews);
     L.err = D.err.as<int>();
     // the detector stack arrives in view chunks (back_chunks) on the copy
     // stream; each chunk is projected back (accumulating into the volume)

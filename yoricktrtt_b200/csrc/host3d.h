@@ -212,29 +212,31 @@ inline void choose_band(int nu, int nv, int &band_rows, int &warps)
   band_rows = rows >= 2 ? (int)rows : 0;
 }
 
-// Bounds for the sweep kernel over the factorised views of a closed-form plan:
+// Bounds for the sweep and gather kernels over the factorised views of a closed-form plan:
 // the detector rows of one voxel column's v footprint, and the part of the
 // detector that any footprint can reach (a volume's shadow seldom fills the
 // detector; the tiles cover no more than it).  rows = 0 where the kernel does
-// not apply: a footprint that is not the cubic's 4 voxels wide (its walk
+// not apply: a footprint that is not the cubic's 4 voxels wide (a walk
 // starts at a zero of the primitive), a source within the volume.
 inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nviews)
 {
-  SweepBounds b = {0, 0, 0, 0, 0};
+  SweepBounds b;
   if (P.hs0 != 2.0) return b;
   double hsv = 0.0, hsu = 0.0, u0 = HUGE_VAL, u1 = -HUGE_VAL, v0 = HUGE_VAL, v1 = -HUGE_VAL;
   for (long n = 0; n < nviews; ++n) {
     const View3D &V = views[n];
-    double wmin = HUGE_VAL, wmax = -HUGE_VAL, dv2 = 0.0, du2 = 0.0;
+    double wmin = HUGE_VAL, wmax = -HUGE_VAL, dv2 = 0.0, du2 = 0.0, dmin = HUGE_VAL, uabs = 0.0;
     for (int c = 0; c < 8; ++c) {
       const double i = (c & 1) ? P.nx - 1 : 0, j = (c & 2) ? P.ny - 1 : 0, k = (c & 4) ? P.nz - 1 : 0;
       double u, v;
       if (P.geom == GEOM_CONE) {
-        const double w = V.o1 * i + V.o2 * j + V.o4, q = V.a4m / (V.d_x * i + V.d_y * j + V.d_c);
+        const double w = V.o1 * i + V.o2 * j + V.o4, d = V.d_x * i + V.d_y * j + V.d_c, q = V.a4m / d;
         v = q * (V.nv_x * i + V.nv_y * j + V.nv_c) + V.b3;
         u = q * (V.nu_x * i + V.nu_y * j + V.nu_z * k + V.nu_c) + V.c3;
         wmin = std::fmin(wmin, w);
         wmax = std::fmax(wmax, w);
+        dmin = std::fmin(dmin, std::fabs(d));
+        uabs = std::fmax(uabs, std::fabs(u - V.c3));
         const double va = (v - V.a8) * P.v_scl, ua = (u - V.a12) * P.u_scl;
         dv2 = std::fmax(dv2, va * va / V.a4sqr);
         du2 = std::fmax(du2, ua * ua / V.a4sqr);
@@ -253,12 +255,18 @@ inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nvi
       const double magn = std::fabs(V.a4m) / std::fmin(std::fabs(wmin), std::fabs(wmax));
       hsv = std::fmax(hsv, P.hs0 * P.h_v0 * magn * std::sqrt(1.0 + dv2));
       hsu = std::fmax(hsu, P.hs0 * P.h_u0 * magn * std::sqrt(1.0 + du2));
+      const double q = std::fabs(V.a4m) / dmin;
+      b.du = std::fmax(b.du, q * std::fabs(V.nu_z));
+      b.dcol = std::fmax(b.dcol, q * std::fabs(V.nu_x) + uabs * std::fabs(V.d_x) / dmin);
     } else {
       hsv = std::fmax(hsv, V.p_hs_v);
       hsu = std::fmax(hsu, V.p_hs_u);
+      b.du = std::fmax(b.du, std::fabs(V.u_z));
+      b.dcol = std::fmax(b.dcol, std::fabs(V.u_x));
     }
   }
-  if (!(hsv > 0.0 && hsv < 1e4 && hsu < 1e4 && u0 > -1e8 && u1 < 1e8 && v0 > -1e8 && v1 < 1e8)) return b;
+  b.hsu = hsu;
+  if (!(hsv > 0.0 && hsv < 1e4 && hsu < 1e4 && b.du < 1e6 && b.dcol < 1e6 && u0 > -1e8 && u1 < 1e8 && v0 > -1e8 && v1 < 1e8)) return b;
   b.rows = (int)std::floor(2.0 * hsv * 1.0001) + 2;
   b.u0 = (int)std::fmin(std::fmax(std::floor(u0 - hsu * 1.0001) - 1.0, 0.0), P.nu);
   b.u1 = (int)std::fmin(std::fmax(std::ceil(u1 + hsu * 1.0001) + 2.0, 0.0), P.nu);

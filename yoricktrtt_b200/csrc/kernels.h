@@ -28,11 +28,13 @@ struct GatePair {
   float w0, w1;
 };
 
-// Bounds of the sweep kernel (sweep_bounds, host3d.h): detector rows of one
-// voxel column (0: the kernel does not apply), reachable cells [u0, u1) and
-// rows [v0, v1).
+// Bounds of the sweep and gather kernels (sweep_bounds, host3d.h): detector
+// rows of one voxel column (0: the kernels do not apply), reachable cells
+// [u0, u1) and rows [v0, v1); cells between neighbouring voxels of a column and
+// between neighbouring columns along i, half support along u.
 struct SweepBounds {
-  int rows, u0, u1, v0, v1;
+  int rows = 0, u0 = 0, u1 = 0, v0 = 0, v1 = 0;
+  double du = 0.0, dcol = 0.0, hsu = 0.0;
 };
 
 struct Fwd3DLaunch {
@@ -48,7 +50,7 @@ struct Fwd3DLaunch {
   int pull = 0;          // closed-form model, nu <= 512: atomic-free band kernel
   int cols = 1;          // closed-form model: 2 = column-pair band kernel
   int tc = 0;            // closed-form model: 1 = tensor-core band kernel (rows chosen by it)
-  SweepBounds sweep = {0, 0, 0, 0, 0};  // closed-form model, rows > 0: sweep kernel
+  SweepBounds sweep;     // closed-form model, rows > 0: sweep kernel
   int *err;              // device error flags
 };
 
@@ -65,6 +67,13 @@ struct Back3DLaunch {
   long gate_stride;
   int factorized;        // 1: column kernel; 0: per-voxel kernel
   const GatePair *pairs = nullptr;  // by view index; non-null: all gates in one pass over the views
+  // closed-form model, sweep.rows > 0: gather kernel, over the views in order
+  // (weights 1), or over the gated views of `order` (sorted by gates) with the
+  // weights of `order_pairs`
+  SweepBounds sweep;
+  const int *order = nullptr;
+  int norder = 0;
+  const GatePair *order_pairs = nullptr;
   int *err;
 };
 
@@ -106,6 +115,29 @@ struct SweepLaunch {
   int band_rows = 0, usplit = 0, utile = 0, split = 0;  // chosen by the launcher
 };
 cudaError_t launch_fwd3d_sweep(const SweepLaunch &L, int G, cudaStream_t st);
+
+// Transpose by neighbouring voxel columns (proj3d_gather.cu; closed-form model,
+// column-factorised views) over views [view_lo, view_hi) (images at
+// sino[view - view_lo]), taken in the order of `order` (all views of the plan)
+// when that is given, with the gate weights of pairs[view].
+struct GatherLaunch {
+  Params3D P;
+  const View3D *views;
+  SweepBounds b;
+  int view_lo, view_hi;
+  const int *order = nullptr;
+  int norder = 0;
+  const GatePair *pairs = nullptr;
+  const float *sino;
+  long sino_view_stride;
+  float *vol;            // column layout, gates stacked, accumulated
+  long gate_stride;
+  int vec4;              // nu % 4 == 0 and 16-byte aligned images
+  int *err;
+  int vsplit = 1, cap = 0;  // chosen by the launcher
+};
+bool gather_fits(const Params3D &P, const SweepBounds &b);
+cudaError_t launch_back3d_gather(const GatherLaunch &L, cudaStream_t st);
 
 // Transpose over orbits of columns under the group's turns, for the groups
 // [g_lo, g_hi) of `groups`.

@@ -541,6 +541,24 @@ cudaError_t launch_fwd3d_fast(const Fwd3DLaunch &L, cudaStream_t st)
 
 cudaError_t launch_back3d_fast(const Back3DLaunch &L, cudaStream_t st)
 {
+  if (L.P.model == MODEL_CUBIC && gather_fits(L.P, L.sweep)) {
+    GatherLaunch A;
+    A.P = L.P;
+    A.views = L.views;
+    A.b = L.sweep;
+    A.view_lo = L.view_lo;
+    A.view_hi = L.view_hi;
+    A.order = L.order;
+    A.norder = L.norder;
+    A.pairs = L.order_pairs;
+    A.sino = L.sino;
+    A.sino_view_stride = L.sino_view_stride;
+    A.vol = L.vol;
+    A.gate_stride = L.gate_stride;
+    A.vec4 = (L.P.nu % 4 == 0 && L.sino_view_stride % 4 == 0 && ((uintptr_t)L.sino & 15) == 0) ? 1 : 0;
+    A.err = L.err;
+    return launch_back3d_gather(A, st);
+  }
   if (L.P.model == MODEL_TABLE)
     return L.P.geom == GEOM_CONE ? back_fast<GEOM_CONE, MODEL_TABLE>(L, st)
                                  : back_fast<GEOM_PARALLEL, MODEL_TABLE>(L, st);
