@@ -195,7 +195,8 @@ extern "C" int trtt_b200_plan3d_create(trtt_b200_plan3d **plan, int geometry,
     if (!pl->hviews[v].factorized) pl->factorized = false;
   }
   choose_band(pl->P.nu, pl->P.nv, pl->band_rows, pl->warps);
-  if (pl->factorized && !cum_footprint) pl->sweep = sweep_bounds(pl->P, pl->hviews.data(), nviews);
+  if (cum_footprint) table_range(pl->P, cum_footprint, size_footprint);
+  if (pl->factorized) pl->sweep = sweep_bounds(pl->P, pl->hviews.data(), nviews);
   if (pl->factorized && !cum_footprint) {
     std::vector<int> lists[3];
     find_view_groups(nx, ny, nviews, xos, xsd, lists);
@@ -881,6 +882,7 @@ int host3d(int geom, double *out, const double *in, long nx, long ny, long nz,
   }
   Params3D P = make_params(geom, nx, ny, nz, s_scl, s_deg, cum_dev, size, step,
                            cum ? coord[0] : 0.0, nu, nv, u_scl, v_scl);
+  if (cum) table_range(P, cum, size);
   std::vector<View3D> hv(nviews);
   bool fact = true;
   for (long v = 0; v < nviews; ++v) {
@@ -977,7 +979,7 @@ int host3d(int geom, double *out, const double *in, long nx, long ny, long nz,
     choose_band((int)nu, (int)nv, rows, warps);
     L.band_rows = rows;
     L.warps = warps;
-    if (P.model == MODEL_CUBIC) L.sweep = sweep_bounds(P, hv.data(), nviews);
+    L.sweep = sweep_bounds(P, hv.data(), nviews);
     L.err = D.err.as<int>();
     const long bands = (nv + rows - 1) / rows;
     const std::vector<long> cb = fwd_chunks(nviews, (nviews + 5) / 6, std::max<long>(1, 2L * D.sms / bands),
@@ -1050,7 +1052,7 @@ int host3d(int geom, double *out, const double *in, long nx, long ny, long nz,
     L.vol = D.vol32.as<float>();
     L.gate_stride = nvox;
     L.factorized = fact ? 1 : 0;
-    if (fact && !cum) L.sweep = sweep_bounds(P, hv.data(), nviews);
+    if (fact) L.sweep = sweep_bounds(P, hv.data(), nviews);
     L.err = D.err.as<int>();
     // the detector stack arrives in view chunks (back_chunks) on the copy
     // stream; each chunk is projected back (accumulating into the volume)

@@ -99,6 +99,16 @@ inline Params3D make_params(int geom, long nx, long ny, long nz, double s_scl, i
   return P;
 }
 
+// Range of slots outside which the table is constant.
+inline void table_range(Params3D &P, const double *cum, long size)
+{
+  long a = 0, b = size - 1;
+  while (a + 1 < size && cum[a + 1] == cum[0]) ++a;
+  while (b > 0 && cum[b - 1] == cum[size - 1]) --b;
+  P.tab0 = (int)(a <= b ? a : 0);
+  P.tab1 = (int)(a <= b ? b : 0);
+}
+
 // Size limits shared by every 3D entry point that takes device arrays:
 // dimensions in [1, 2^30) (int indices in the kernels), one volume slice
 // below 2^31 voxels and the whole volume below 2^40.  Returns nullptr when
@@ -221,11 +231,13 @@ inline void choose_band(int nu, int nv, int &band_rows, int &warps)
 inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nviews)
 {
   SweepBounds b;
-  if (P.hs0 != 2.0) return b;
+  if (P.model == MODEL_CUBIC && P.hs0 != 2.0) return b;
+  double hmin = HUGE_VAL;
   double hsv = 0.0, hsu = 0.0, u0 = HUGE_VAL, u1 = -HUGE_VAL, v0 = HUGE_VAL, v1 = -HUGE_VAL;
   for (long n = 0; n < nviews; ++n) {
     const View3D &V = views[n];
     double wmin = HUGE_VAL, wmax = -HUGE_VAL, dv2 = 0.0, du2 = 0.0, dmin = HUGE_VAL, uabs = 0.0;
+    int dneg = 0;  // corners behind the plane where u and v diverge
     for (int c = 0; c < 8; ++c) {
       const double i = (c & 1) ? P.nx - 1 : 0, j = (c & 2) ? P.ny - 1 : 0, k = (c & 4) ? P.nz - 1 : 0;
       double u, v;
@@ -236,6 +248,7 @@ inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nvi
         wmin = std::fmin(wmin, w);
         wmax = std::fmax(wmax, w);
         dmin = std::fmin(dmin, std::fabs(d));
+        dneg += d < 0.0;
         uabs = std::fmax(uabs, std::fabs(u - V.c3));
         const double va = (v - V.a8) * P.v_scl, ua = (u - V.a12) * P.u_scl;
         dv2 = std::fmax(dv2, va * va / V.a4sqr);
@@ -250,15 +263,17 @@ inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nvi
       v1 = std::fmax(v1, v);
     }
     if (P.geom == GEOM_CONE) {
-      if (!(wmin * wmax > 0.0)) return b;
+      if (!(wmin * wmax > 0.0) || (P.model == MODEL_TABLE && dneg % 8 != 0)) return b;
       // nearest corner: largest magnification; outermost: largest obliquity
       const double magn = std::fabs(V.a4m) / std::fmin(std::fabs(wmin), std::fabs(wmax));
       hsv = std::fmax(hsv, P.hs0 * P.h_v0 * magn * std::sqrt(1.0 + dv2));
       hsu = std::fmax(hsu, P.hs0 * P.h_u0 * magn * std::sqrt(1.0 + du2));
+      hmin = std::fmin(hmin, P.h_u0 * std::fabs(V.a4m) / std::fmax(std::fabs(wmin), std::fabs(wmax)));
       const double q = std::fabs(V.a4m) / dmin;
       b.du = std::fmax(b.du, q * std::fabs(V.nu_z));
       b.dcol = std::fmax(b.dcol, q * std::fabs(V.nu_x) + uabs * std::fabs(V.d_x) / dmin);
     } else {
+      hmin = std::fmin(hmin, V.p_h_u);
       hsv = std::fmax(hsv, V.p_hs_v);
       hsu = std::fmax(hsu, V.p_hs_u);
       b.du = std::fmax(b.du, std::fabs(V.u_z));
@@ -266,6 +281,10 @@ inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nvi
     }
   }
   b.hsu = hsu;
+  // table: slots along a footprint are 32-bit integers
+  if (P.model == MODEL_TABLE && !(hmin > 0.0 && (2.0 * hsu + 20.0 + std::fabs(P.coord0)) / (hmin * P.step) < 1e9 &&
+                                  (2.0 * P.hs0 + std::fabs(P.coord0)) / P.step < 1e9))
+    return b;
   if (!(hsv > 0.0 && hsv < 1e4 && hsu < 1e4 && b.du < 1e6 && b.dcol < 1e6 && u0 > -1e8 && u1 < 1e8 && v0 > -1e8 && v1 < 1e8)) return b;
   b.rows = (int)std::floor(2.0 * hsv * 1.0001) + 2;
   b.u0 = (int)std::fmin(std::fmax(std::floor(u0 - hsu * 1.0001) - 1.0, 0.0), P.nu);

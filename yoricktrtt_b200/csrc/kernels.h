@@ -50,7 +50,7 @@ struct Fwd3DLaunch {
   int pull = 0;          // closed-form model, nu <= 512: atomic-free band kernel
   int cols = 1;          // closed-form model: 2 = column-pair band kernel
   int tc = 0;            // closed-form model: 1 = tensor-core band kernel (rows chosen by it)
-  SweepBounds sweep;     // closed-form model, rows > 0: sweep kernel
+  SweepBounds sweep;     // rows > 0: sweep kernel
   int *err;              // device error flags
 };
 
@@ -67,7 +67,7 @@ struct Back3DLaunch {
   long gate_stride;
   int factorized;        // 1: column kernel; 0: per-voxel kernel
   const GatePair *pairs = nullptr;  // by view index; non-null: all gates in one pass over the views
-  // closed-form model, sweep.rows > 0: gather kernel, over the views in order
+  // sweep.rows > 0: gather kernel, over the views in order
   // (weights 1), or over the gated views of `order` (sorted by gates) with the
   // weights of `order_pairs`
   SweepBounds sweep;
@@ -98,9 +98,9 @@ struct GroupFwdLaunch {
   int *err;
 };
 
-// Direct projector by sweeps over image lines (proj3d_sweep.cu; closed-form
-// model, column-factorised views) of `count` view groups of `groups` (4 view
-// indices each) or, with groups null, `count` single views; at most 65535.
+// Direct projector by sweeps over image lines (proj3d_sweep.cu; column-factorised
+// views) of `count` view groups of `groups` (4 view indices each; closed-form
+// model) or, with groups null, `count` single views; at most 65535.
 struct SweepLaunch {
   Params3D P;
   const View3D *views;
@@ -116,8 +116,8 @@ struct SweepLaunch {
 };
 cudaError_t launch_fwd3d_sweep(const SweepLaunch &L, int G, cudaStream_t st);
 
-// Transpose by neighbouring voxel columns (proj3d_gather.cu; closed-form model,
-// column-factorised views) over views [view_lo, view_hi) (images at
+// Transpose by neighbouring voxel columns (proj3d_gather.cu; column-factorised
+// views) over views [view_lo, view_hi) (images at
 // sino[view - view_lo]), taken in the order of `order` (all views of the plan)
 // when that is given, with the gate weights of pairs[view].
 struct GatherLaunch {

@@ -1,5 +1,8 @@
 // proj3d_fast.cu -- per-view 3D projector pair for column-factorised views
-// (circular orbits), both footprint models.
+// (circular orbits), both footprint models: the launchers' choice between the
+// sweep and gather kernels (proj3d_sweep.cu, proj3d_gather.cu) and the general
+// ones here, which serve what those do not take: a footprint that is not the
+// cubic's, a source within the volume, long tables, asked-for band shapes.
 //
 // Direct: one CTA per (band of detector rows, view) accumulates the band in
 // shared memory; its warps pull 32-column chunks, build each hit column's
@@ -18,6 +21,7 @@
 #include <cstdint>
 
 #include "fast3d_items.cuh"
+#include "table3d.cuh"
 #include "kernels.h"
 
 namespace trtt {
@@ -522,7 +526,7 @@ static cudaError_t back_fast(const Back3DLaunch &L, cudaStream_t st)
 cudaError_t launch_fwd3d_fast(const Fwd3DLaunch &L, cudaStream_t st)
 {
   if (L.tc && L.P.model == MODEL_CUBIC) return launch_fwd3d_tc(L, st);
-  if (L.P.model == MODEL_CUBIC && L.sweep.rows > 0 && L.nviews <= 65535) {
+  if (L.sweep.rows > 0 && L.nviews <= 65535 && (L.P.model == MODEL_CUBIC || L.P.tab1 - L.P.tab0 < kTableSlots)) {
     SweepLaunch S;
     S.P = L.P;
     S.views = L.views;
@@ -541,7 +545,7 @@ cudaError_t launch_fwd3d_fast(const Fwd3DLaunch &L, cudaStream_t st)
 
 cudaError_t launch_back3d_fast(const Back3DLaunch &L, cudaStream_t st)
 {
-  if (L.P.model == MODEL_CUBIC && gather_fits(L.P, L.sweep)) {
+  if (gather_fits(L.P, L.sweep)) {
     GatherLaunch A;
     A.P = L.P;
     A.views = L.views;

@@ -1,6 +1,7 @@
-// proj3d_gather.cu -- transpose 3D projection of column-factorised views,
-// closed-form model, view by view: one warp gathers four neighbouring voxel
-// columns (a k range of each) over all views.
+// proj3d_gather.cu -- transpose 3D projection of column-factorised views
+// (closed-form footprint; tabulated footprint with table3d.cuh), view by view:
+// one warp gathers four neighbouring voxel columns (a k range of each) over all
+// views.
 //
 // Per view the warp
 //   * builds the four columns' v-collapsed detector profiles Q_g[u] = sum_v
@@ -21,7 +22,7 @@
 // halves the shared memory loads and a row load serves four columns, against
 // one warp per column that walked each voxel for itself.  Measured, before ->
 // after: cone 100 x 92 x 75 voxels x 61 views 1.07 -> 0.354 ms, parallel 97^2
-// x 83 x 75 views 1.04 -> 0.731 ms, one cone view of 128^3 75 -> 36 us, 128^2
+// x 83 x 75 views 1.04 -> 0.64 ms, one cone view of 128^3 75 -> 36 us, 128^2
 // x 64 x 10 gates x 400 views 9.04 -> 5.10 ms.  View groups keep
 // k_back3d_group, whose footprint serves two or four views: at 128^3 x 90
 // views 1.36 ms against 1.67 here, and 1.58 with grouped columns in this form;
@@ -36,9 +37,8 @@ namespace trtt {
 
 namespace {
 
-constexpr int kWarps = 8, kH = 8, kNC = 4;  // warps per CTA, lanes per column, columns per warp
-constexpr int kBatch = 32 / kNC;            // views whose column records are built together
-constexpr int kTabRows = 32;                // detector rows per weight table
+constexpr int kH = 8, kNC = 4;    // lanes per column, columns per warp
+constexpr int kTabRows = 32;      // detector rows per weight table
 
 struct GatherCol {
   long long A, B;             // 32.32 position of voxel 0 and step per voxel
@@ -54,9 +54,19 @@ struct GatherCol {
 // Shared memory of one warp: records, weight table, four profile rows of
 // `cap` cells with zeros before and after them.
 __host__ __device__ constexpr size_t gather_row(int cap) { return (size_t)((cap + 2 * kSweepGuard + 3) & ~3); }
-__host__ __device__ constexpr size_t gather_warp_bytes(int cap)
+template <int MODEL> struct GatherRec {
+  using T = GatherCol;
+  static constexpr int warps = 8;          // per CTA
+  static constexpr int batch = 32 / kNC;   // views whose column records are built together
+};
+template <> struct GatherRec<MODEL_TABLE> {
+  using T = TableCol;
+  static constexpr int warps = 24;
+  static constexpr int batch = 16 / kNC;
+};
+template <int MODEL> __host__ __device__ constexpr size_t gather_warp_bytes(int cap)
 {
-  return 32 * sizeof(GatherCol) + sizeof(float2) * kTabRows * kNC + sizeof(float) * kNC * gather_row(cap);
+  return GatherRec<MODEL>::batch * kNC * sizeof(typename GatherRec<MODEL>::T) + sizeof(float2) * kTabRows * kNC + sizeof(float) * kNC * gather_row(cap);
 }
 
 template <int GEOM>
@@ -104,6 +114,26 @@ __device__ __forceinline__ void gather_record(const Params3D &P, const View3D &V
   r.view = 0;
 }
 
+// The same of the tabulated footprint.
+template <int GEOM>
+__device__ __forceinline__ void gather_record(const Params3D &P, const View3D &V, int i, int j, int k0, int k1,
+                                              TableCol &r, int *__restrict__ err)
+{
+  double A, B, hsm, sp;
+  if (!table_column<GEOM>(P, V, i, j, r, A, B, hsm, sp, err)) {
+    r.n = 0;
+    return;
+  }
+  const double ua = fma(B, (double)k0, A), ub = fma(B, (double)(k1 - 1), A);
+  const double lo = fmin(ua, ub) - hsm - 1.0, hi = fmax(ua, ub) + hsm + 2.0;
+  if (!(hi > 0.0 && lo < (double)P.nu)) return;
+  const int c0 = (int)fmax(lo, 0.0), c1 = (int)fmin(hi, (double)P.nu);
+  if (c0 >= c1) return;
+  r.c0 = c0;
+  r.c1 = c1;
+  r.view = 0;
+}
+
 // acc += term, compensated.
 __device__ __forceinline__ void kahan(float &acc, float &cmp, float term)
 {
@@ -112,10 +142,20 @@ __device__ __forceinline__ void kahan(float &acc, float &cmp, float term)
   acc = t;
 }
 
-template <int GEOM, int PP, bool GATED>
-__global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d_gather(const GatherLaunch A)
+template <int GEOM, int PP, bool GATED, int MODEL>
+__global__ void __launch_bounds__(32 * GatherRec<MODEL>::warps, MODEL == MODEL_TABLE ? 1 : (GATED || PP > 3 ? 2 : 3))
+k_back3d_gather(const GatherLaunch A)
 {
-  extern __shared__ __align__(16) unsigned char smem[];
+  extern __shared__ __align__(16) unsigned char smem_all[];
+  using Rec = typename GatherRec<MODEL>::T;
+  constexpr int kWarps = GatherRec<MODEL>::warps, kBatch = GatherRec<MODEL>::batch;
+  TableSh T{};
+  unsigned char *smem = smem_all;
+  if constexpr (MODEL == MODEL_TABLE) {
+    table_load(A.P, reinterpret_cast<double *>(smem_all), T);
+    smem += table_bytes(A.P);
+    __syncthreads();
+  }
   constexpr int NA = GATED ? 2 : 1;  // sums per voxel: the current gates
   const Params3D &P = A.P;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane / kH, lig = lane & (kH - 1);
@@ -127,10 +167,10 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
   const int col_i = i0 + grp;
   const int pb = blockIdx.y * (kH * PP);
   const int k0 = 2 * pb, k1 = min(k0 + 2 * kH * PP, nz);
-  const size_t wb = gather_warp_bytes(A.cap);
+  const size_t wb = gather_warp_bytes<MODEL>(A.cap);
   const int qrow = (int)gather_row(A.cap);
-  GatherCol *recs = reinterpret_cast<GatherCol *>(smem + warp * wb);
-  float2 *wtab = reinterpret_cast<float2 *>(recs + 32);
+  Rec *recs = reinterpret_cast<Rec *>(smem + warp * wb);
+  float2 *wtab = reinterpret_cast<float2 *>(recs + kBatch * kNC);
   float *Q = reinterpret_cast<float *>(wtab + kTabRows * kNC);
   for (int t = lane; t < kNC * qrow; t += 32) Q[t] = 0.f;
   __syncwarp();
@@ -151,9 +191,11 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
       float *dst = A.vol + (long)g * A.gate_stride + ((long)j * nx + col_i) * nz;
 #pragma unroll
       for (int i = 0; i < PP; ++i) {
-        const int k = 2 * (pb + lig + kH * i);
+        // the lane's voxels: pairs of neighbours, or (table) every kH-th
+        const int k = MODEL == MODEL_TABLE ? k0 + lig + 2 * kH * i : 2 * (pb + lig + kH * i);
+        const int k2 = MODEL == MODEL_TABLE ? k + kH : k + 1;
         if (k < nz) dst[k] += acc[a][i][0] - cmp[a][i][0];
-        if (k + 1 < nz) dst[k + 1] += acc[a][i][1] - cmp[a][i][1];
+        if (k2 < nz) dst[k2] += acc[a][i][1] - cmp[a][i][1];
       }
     }
 #pragma unroll
@@ -170,14 +212,14 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
     // ---- records of kBatch views x kNC columns ---------------------------
     {
       const int n = vb + lane / kNC, ci = i0 + lane % kNC;
-      GatherCol r;
+      Rec r;
       r.view = -1;
       r.n = 0;
       r.c0 = INT_MAX;
       r.c1 = INT_MIN;
-      r.steps = 0;
       r.lo = 0;
-      if (n < nview && ci < nx) {
+      if constexpr (MODEL == MODEL_CUBIC) r.steps = 0;
+      if (n < nview && ci < nx && lane < kBatch * kNC) {
         const int v = A.order ? A.order[n] : A.view_lo + n;
         if (v >= A.view_lo && v < A.view_hi) {
           gather_record<GEOM>(P, A.views[v], ci, j, k0, k1, r, A.err);
@@ -185,19 +227,18 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
         }
       }
       __syncwarp();
-      recs[lane] = r;
+      if (lane < kBatch * kNC) recs[lane] = r;
       __syncwarp();
     }
     const int cnt = min(kBatch, nview - vb);
 #pragma unroll 1
     for (int b = 0; b < cnt; ++b) {
-      const GatherCol &r = recs[b * kNC + grp];
+      const Rec &r = recs[b * kNC + grp];
       const bool on = r.view >= 0;
       const int view = __reduce_max_sync(FULLM, r.view);
       if (view < 0) continue;
       const int r0 = __reduce_min_sync(FULLM, on ? r.lo : INT_MAX), r1 = __reduce_max_sync(FULLM, on ? r.lo + r.n : INT_MIN);
       int c0 = __reduce_min_sync(FULLM, r.c0) & ~3, c1 = __reduce_max_sync(FULLM, r.c1);
-      const int steps = __reduce_max_sync(FULLM, r.steps);
       if (A.vec4) c1 = (c1 + 3) & ~3;
       if (c1 - c0 > A.cap) {  // more cells than the launcher's bound: never in a correct run
         if (lane == 0) atomicOr(A.err, TRTT_ERR_BAD_INDEX);
@@ -235,14 +276,18 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
       for (int rb = r0; rb < r1; rb += kTabRows) {
         const int nr = min(kTabRows, r1 - rb);
         for (int e = lane; e < nr * kNC; e += 32) {
-          const GatherCol &o = recs[b * kNC + e % kNC];
+          const Rec &o = recs[b * kNC + e % kNC];
           const int l = rb + e / kNC - o.lo;
           float w = 0.f;
           if (o.view >= 0 && l >= 0 && l < o.n) {
-            AxisCubic ax;
-            ax.start = o.vstart;
-            ax.inc = o.vinc;
-            w = edge_cubic(ax, l + 1) - edge_cubic(ax, l);
+            if constexpr (MODEL == MODEL_TABLE) {
+              w = table_weight_v(T, o, l);
+            } else {
+              AxisCubic ax;
+              ax.start = o.vstart;
+              ax.inc = o.vinc;
+              w = edge_cubic(ax, l + 1) - edge_cubic(ax, l);
+            }
           }
           wtab[e] = f2(w);
         }
@@ -322,70 +367,7 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
       }
       __syncwarp();
       // ---- gather ----------------------------------------------------------
-      const long long B = r.B, B2 = 2 * B;
-      const bool up = B >= 0;
-      float h_c = 0.f, rho_c = 0.f, inv_den = 0.f;
-      if constexpr (GEOM == GEOM_CONE) {
-        h_c = r.h;
-        rho_c = on ? r.rho : 0.f;
-        inv_den = r.inv_den;
-      } else {
-        h_c = (float)A.views[view].p_hs_u;
-        rho_c = on ? (float)A.views[view].p_rho0 : 0.f;
-      }
-      const float a12 = (float)A.views[view].a12, pscl = GEOM == GEOM_CONE ? 0.f : (float)A.views[view].p_scl_u;
-      long long ue = r.A + B2 * (pb + lig);
-      const float *row = Q + grp * qrow + kSweepGuard;
-      const int rmax = c1 - c0 + kSweepGuard - 2 * steps;  // last start of a walk
-#pragma unroll
-      for (int i = 0; i < PP; ++i) {
-        const long long uo = ue + B, ua = up ? ue : uo, uc = up ? uo : ue;
-        ue += B2 * kH;
-        const int Ia = (int)(ua >> 32), Ic = (int)(uc >> 32);
-        const float2 ph = make_float2(__uint_as_float(((unsigned)ua >> 9) | 0x3f800000u) - 1.0f,
-                                      __uint_as_float(((unsigned)uc >> 9) | 0x3f800000u) - 1.0f);
-        float2 scl, rho;
-        float hs;
-        if constexpr (GEOM == GEOM_CONE) {
-          const float2 uca = mul2(add2(make_float2((float)Ia, (float)Ic), add2(ph, f2(-a12))), f2((float)P.u_scl));
-          const float2 du2 = fma2(mul2(uca, uca), f2(inv_den), f2(1.0f));
-          const float2 dlt = mul2(du2, make_float2(rsqrt_ftz(du2.x), rsqrt_ftz(du2.y)));
-          const float2 h = mul2(dlt, f2(h_c));
-          scl = make_float2(rcp_ftz(h.x), rcp_ftz(h.y));
-          rho = mul2(dlt, f2(rho_c));
-          hs = (float)P.hs0 * h.x;
-        } else {
-          scl = f2(pscl);
-          rho = f2(rho_c);
-          hs = h_c;
-        }
-        const float fm = __fadd_rd(ph.x - hs, 12582912.0f);
-        const int f = Ia + (__float_as_int(fm) - 0x4B400000);
-        const float2 x1 = mul2(add2(make_float2(fm - 12582911.0f, (float)(f + 1 - Ic)),
-                                    make_float2(-ph.x, -ph.y)), scl);
-        // a walk that would start before the guard or end behind it touches no
-        // cell of the detector: it is moved into the zeros in front
-        int rel = f - c0;
-        const bool in = on && rel >= -kSweepGuard && rel <= rmax;
-        rel = in ? rel : -kSweepGuard;
-        const int st = in ? steps : 0;
-        const float *cell = row + rel;
-        float ax = x1.x, cx = x1.y, pa = -0.5f, pc = -0.5f, sa = 0.f, sc = 0.f;
-#pragma unroll 1
-        for (int l = 0; l < st; ++l) {
-          const float y0 = cell[0], y1 = cell[1];
-          const float ay = ax + scl.x, cy = cx + scl.y;
-          const float a1 = cubic_odd(ax), q1 = cubic_odd(cx), a2 = cubic_odd(ay), q2 = cubic_odd(cy);
-          sa = fmaf(a2 - a1, y1, fmaf(a1 - pa, y0, sa));
-          sc = fmaf(q2 - q1, y1, fmaf(q1 - pc, y0, sc));
-          pa = a2;
-          pc = q2;
-          ax = ay + scl.x;
-          cx = cy + scl.y;
-          cell += 2;
-        }
-        const float ta = in ? sa * rho.x : 0.f, tc = in ? sc * rho.y : 0.f;
-        const float te = up ? ta : tc, to = up ? tc : ta;
+      auto add = [&](int i, float te, float to) {
         if (GATED) {
           kahan(acc[0][i][0], cmp[0][i][0], wa * te);
           kahan(acc[0][i][1], cmp[0][i][1], wa * to);
@@ -394,6 +376,132 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
         } else {
           kahan(acc[0][i][0], cmp[0][i][0], te);
           kahan(acc[0][i][1], cmp[0][i][1], to);
+        }
+      };
+      if constexpr (MODEL == MODEL_TABLE) {
+        const float *row = Q + grp * qrow + kSweepGuard;
+        const View3D &V = A.views[view];
+#pragma unroll
+        for (int i = 0; i < PP; ++i) {
+          // two voxels at a time: their chains of FP64 operations overlap
+          TableVox v, w;
+          table_voxel<GEOM>(P, V, T, r, table_kc<GEOM>(V, k0 + lig + kH * 2 * i), c0, c1, v);
+          table_voxel<GEOM>(P, V, T, r, table_kc<GEOM>(V, k0 + lig + kH * (2 * i + 1)), c0, c1, w);
+          if (!on) v.n = w.n = 0;
+          const int steps = (__reduce_max_sync(FULLM, max(v.n > 0 ? v.s + v.n : 0, w.n > 0 ? w.s + w.n : 0)) + 1) & ~1;
+          // walks that touch no cell go over the zeros in front; walks that would
+          // leave the guards (none where a footprint fits them) only load their cells
+          int rv = v.n > 0 ? v.f - c0 : -kSweepGuard, rw = w.n > 0 ? w.f - c0 : -kSweepGuard;
+          const int rmax = c1 - c0 + kSweepGuard - steps;
+          const bool safe = __all_sync(FULLM, min(rv, rw) >= -kSweepGuard && max(rv, rw) <= rmax);
+          double lv = (double)(-v.l0), ev = table_at(T, dadd(v.start, dmul(lv, v.inc)));
+          double lw = (double)(-w.l0), ew = table_at(T, dadd(w.start, dmul(lw, w.inc)));
+          float sv = 0.f, sw = 0.f;
+          const float *cv = row + rv, *cw = row + rw;
+          if (safe) {
+            int tv = -v.s, tw = -w.s;
+#pragma unroll 1
+            for (int t = 0; t < steps; t += 2) {
+              const double v1 = table_at(T, dadd(v.start, dmul(lv + 1.0, v.inc)));
+              const double w1 = table_at(T, dadd(w.start, dmul(lw + 1.0, w.inc)));
+              lv += 2.0;
+              lw += 2.0;
+              const double v2 = table_at(T, dadd(v.start, dmul(lv, v.inc)));
+              const double w2 = table_at(T, dadd(w.start, dmul(lw, w.inc)));
+              const float y0 = cv[0], z0 = cw[0], y1 = cv[1], z1 = cw[1];
+              if ((unsigned)tv < (unsigned)v.n) sv = fmaf((float)(v1 - ev), y0, sv);
+              if ((unsigned)tw < (unsigned)w.n) sw = fmaf((float)(w1 - ew), z0, sw);
+              if ((unsigned)(tv + 1) < (unsigned)v.n) sv = fmaf((float)(v2 - v1), y1, sv);
+              if ((unsigned)(tw + 1) < (unsigned)w.n) sw = fmaf((float)(w2 - w1), z1, sw);
+              ev = v2;
+              ew = w2;
+              cv += 2;
+              cw += 2;
+              tv += 2;
+              tw += 2;
+            }
+          } else {
+#pragma unroll 1
+            for (int t = 0; t < steps; ++t) {
+              lv += 1.0;
+              lw += 1.0;
+              const double v1 = table_at(T, dadd(v.start, dmul(lv, v.inc)));
+              const double w1 = table_at(T, dadd(w.start, dmul(lw, w.inc)));
+              if ((unsigned)(t - v.s) < (unsigned)v.n) sv = fmaf((float)(v1 - ev), cv[t], sv);
+              if ((unsigned)(t - w.s) < (unsigned)w.n) sw = fmaf((float)(w1 - ew), cw[t], sw);
+              ev = v1;
+              ew = w1;
+            }
+          }
+          add(i, v.n > 0 ? sv * v.rho : 0.f, w.n > 0 ? sw * w.rho : 0.f);
+        }
+      } else {
+        const int steps = __reduce_max_sync(FULLM, r.steps);
+        const long long B = r.B, B2 = 2 * B;
+        const bool up = B >= 0;
+        float h_c = 0.f, rho_c = 0.f, inv_den = 0.f;
+        if constexpr (GEOM == GEOM_CONE) {
+          h_c = r.h;
+          rho_c = on ? r.rho : 0.f;
+          inv_den = r.inv_den;
+        } else {
+          h_c = (float)A.views[view].p_hs_u;
+          rho_c = on ? (float)A.views[view].p_rho0 : 0.f;
+        }
+        const float a12 = (float)A.views[view].a12, pscl = GEOM == GEOM_CONE ? 0.f : (float)A.views[view].p_scl_u;
+        long long ue = r.A + B2 * (pb + lig);
+        const float *row = Q + grp * qrow + kSweepGuard;
+        const int rmax = c1 - c0 + kSweepGuard - 2 * steps;  // last start of a walk
+  #pragma unroll
+        for (int i = 0; i < PP; ++i) {
+          const long long uo = ue + B, ua = up ? ue : uo, uc = up ? uo : ue;
+          ue += B2 * kH;
+          const int Ia = (int)(ua >> 32), Ic = (int)(uc >> 32);
+          const float2 ph = make_float2(__uint_as_float(((unsigned)ua >> 9) | 0x3f800000u) - 1.0f,
+                                        __uint_as_float(((unsigned)uc >> 9) | 0x3f800000u) - 1.0f);
+          float2 scl, rho;
+          float hs;
+          if constexpr (GEOM == GEOM_CONE) {
+            const float2 uca = mul2(add2(make_float2((float)Ia, (float)Ic), add2(ph, f2(-a12))), f2((float)P.u_scl));
+            const float2 du2 = fma2(mul2(uca, uca), f2(inv_den), f2(1.0f));
+            const float2 dlt = mul2(du2, make_float2(rsqrt_ftz(du2.x), rsqrt_ftz(du2.y)));
+            const float2 h = mul2(dlt, f2(h_c));
+            scl = make_float2(rcp_ftz(h.x), rcp_ftz(h.y));
+            rho = mul2(dlt, f2(rho_c));
+            hs = (float)P.hs0 * h.x;
+          } else {
+            scl = f2(pscl);
+            rho = f2(rho_c);
+            hs = h_c;
+          }
+          const float fm = __fadd_rd(ph.x - hs, 12582912.0f);
+          const int f = Ia + (__float_as_int(fm) - 0x4B400000);
+          const float2 x1 = mul2(add2(make_float2(fm - 12582911.0f, (float)(f + 1 - Ic)),
+                                      make_float2(-ph.x, -ph.y)), scl);
+          // a walk that would start before the guard or end behind it touches no
+          // cell of the detector: it is moved into the zeros in front
+          int rel = f - c0;
+          const bool in = on && rel >= -kSweepGuard && rel <= rmax;
+          rel = in ? rel : -kSweepGuard;
+          const int st = in ? steps : 0;
+          const float *cell = row + rel;
+          float ax = x1.x, cx = x1.y, pa = -0.5f, pc = -0.5f, sa = 0.f, sc = 0.f;
+  #pragma unroll 1
+          for (int l = 0; l < st; ++l) {
+            const float y0 = cell[0], y1 = cell[1];
+            const float ay = ax + scl.x, cy = cx + scl.y;
+            const float a1 = cubic_odd(ax), q1 = cubic_odd(cx), a2 = cubic_odd(ay), q2 = cubic_odd(cy);
+            sa = fmaf(a2 - a1, y1, fmaf(a1 - pa, y0, sa));
+            sc = fmaf(q2 - q1, y1, fmaf(q1 - pc, y0, sc));
+            pa = a2;
+            pc = q2;
+            ax = ay + scl.x;
+            cx = cy + scl.y;
+            cell += 2;
+          }
+          const float ta = in ? sa * rho.x : 0.f, tc = in ? sc * rho.y : 0.f;
+          const float te = up ? ta : tc, to = up ? tc : ta;
+          add(i, te, to);
         }
       }
       __syncwarp();
@@ -434,22 +542,32 @@ __global__ void __launch_bounds__(32 * kWarps, GATED || PP > 3 ? 2 : 3) k_back3d
   }
 }
 
-template <int GEOM, int PP>
+template <int GEOM, int PP, int MODEL>
 cudaError_t launch(GatherLaunch L, cudaStream_t st)
 {
+  constexpr int kWarps = GatherRec<MODEL>::warps, kBatch = GatherRec<MODEL>::batch;
   const int pairs = (L.P.nz + 1) / 2, chunks = (pairs + kH * PP - 1) / (kH * PP);
   const long groups = (long)((L.P.nx + kNC - 1) / kNC) * L.P.ny;
-  // warps that share the views of a column group: until there are 24 per SM,
-  // each with at least 8 views
+  // warps that share the views of a column group, each with at least a batch
   L.vsplit = 1;
-  if (!L.pairs)
-    while (L.vsplit < kWarps && groups * chunks * L.vsplit < 148 * 24 && L.view_hi - L.view_lo >= 2 * kBatch * L.vsplit)
-      L.vsplit *= 2;
+  if (!L.pairs) {
+    const long slots = 148 * (MODEL == MODEL_TABLE ? 1 : (PP > 3 ? 2 : 3));
+    double best = 1e300;
+    for (int s = 1; s <= 8 && (s == 1 || L.view_hi - L.view_lo >= kBatch * s); s *= 2) {
+      // waves of CTAs (and a part for the uneven ends) times the work of each
+      const long ctas = (groups * s + kWarps - 1) / kWarps * chunks;
+      const double cost = ((double)((ctas + slots - 1) / slots) + 0.3) * (1.0 / s + 0.04);
+      if (cost < 0.97 * best) {
+        best = cost;
+        L.vsplit = s;
+      }
+    }
+  }
   // cells of a k range: its voxels' positions in four neighbouring columns and
   // their half supports
   const double len = L.b.du * 2 * kH * PP + L.b.dcol * (kNC - 1) + 2.0 * L.b.hsu + 16.0;
   L.cap = len < (double)L.P.nu ? (int)len : (L.P.nu + 3) & ~3;
-  const size_t smem = std::max(kWarps * gather_warp_bytes(L.cap), sizeof(float2) * 2 * PP * 32 * kWarps);
+  const size_t smem = table_bytes(L.P) + std::max(kWarps * gather_warp_bytes<MODEL>(L.cap), sizeof(float2) * 2 * PP * 32 * kWarps);
   if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
   const dim3 grid((unsigned)((groups * L.vsplit + kWarps - 1) / kWarps), (unsigned)chunks);
   auto go = [&](auto kern) {
@@ -458,34 +576,35 @@ cudaError_t launch(GatherLaunch L, cudaStream_t st)
     kern<<<grid, 32 * kWarps, smem, st>>>(L);
     return cudaGetLastError();
   };
-  return L.pairs ? go(k_back3d_gather<GEOM, PP, true>) : go(k_back3d_gather<GEOM, PP, false>);
+  return L.pairs ? go(k_back3d_gather<GEOM, PP, true, MODEL>) : go(k_back3d_gather<GEOM, PP, false, MODEL>);
 }
 
-// Voxel pairs per lane: the fewest lanes times passes over the column, longer
-// ranges first (each range builds its own profiles).
-int pairs_per_lane(int nz)
+// Voxel pairs per lane (at most `most`): the fewest passes over the column's
+// pairs; each range of k also builds its own profiles, about a pass's work.
+int pairs_per_lane(int nz, int most)
 {
   const int pairs = (nz + 1) / 2;
-  int best = 1, slots = INT_MAX;
-  for (int pp = 5; pp >= 1; --pp) {
-    const int s = (pairs + kH * pp - 1) / (kH * pp) * pp;
-    if (s < slots) {
-      slots = s;
+  int best = 1, cost = INT_MAX;
+  for (int pp = most; pp >= 1; --pp) {
+    const int s = (pairs + kH * pp - 1) / (kH * pp) * (pp + 1);
+    if (s < cost) {
+      cost = s;
       best = pp;
     }
   }
   return best;
 }
 
-template <int GEOM>
+template <int GEOM, int MODEL>
 cudaError_t launch_geom(const GatherLaunch &L, cudaStream_t st)
 {
-  switch (pairs_per_lane(L.P.nz)) {
-    case 1: return launch<GEOM, 1>(L, st);
-    case 2: return launch<GEOM, 2>(L, st);
-    case 3: return launch<GEOM, 3>(L, st);
-    case 4: return launch<GEOM, 4>(L, st);
-    default: return launch<GEOM, 5>(L, st);
+  // (gated sums of the tabulated footprint: beyond 2 pairs the registers spill)
+  switch (pairs_per_lane(L.P.nz, MODEL == MODEL_TABLE && L.pairs ? 2 : 5)) {
+    case 1: return launch<GEOM, 1, MODEL>(L, st);
+    case 2: return launch<GEOM, 2, MODEL>(L, st);
+    case 3: return launch<GEOM, 3, MODEL>(L, st);
+    case 4: return launch<GEOM, 4, MODEL>(L, st);
+    default: return launch<GEOM, 5, MODEL>(L, st);
   }
 }
 
@@ -493,16 +612,23 @@ cudaError_t launch_geom(const GatherLaunch &L, cudaStream_t st)
 
 bool gather_fits(const Params3D &P, const SweepBounds &b)
 {
-  const double len = b.du * 2 * kH * pairs_per_lane(P.nz) + b.dcol * (kNC - 1) + 2.0 * b.hsu + 16.0;
+  const double len = b.du * 2 * kH * pairs_per_lane(P.nz, 5) + b.dcol * (kNC - 1) + 2.0 * b.hsu + 16.0;
   const int cap = len < (double)P.nu ? (int)len : (P.nu + 3) & ~3;
-  return b.rows > 0 && kWarps * gather_warp_bytes(cap) <= 113 * 1024 && (P.nz + 1) / 2 / kH < 65535 &&
+  if (P.model == MODEL_TABLE)
+    return b.rows > 0 && table_slots(P) <= kTableSlots && (P.nz + 1) / 2 / kH < 65535 &&
+           table_bytes(P) + GatherRec<MODEL_TABLE>::warps * gather_warp_bytes<MODEL_TABLE>(cap) <= 227 * 1024;
+  return b.rows > 0 && GatherRec<MODEL_CUBIC>::warps * gather_warp_bytes<MODEL_CUBIC>(cap) <= 113 * 1024 && (P.nz + 1) / 2 / kH < 65535 &&
          2.0 * b.hsu + b.du + 4.0 < 2.0 * kSweepGuard - 16.0;
 }
 
 cudaError_t launch_back3d_gather(const GatherLaunch &L, cudaStream_t st)
 {
   if (L.view_hi <= L.view_lo) return cudaSuccess;
-  return L.P.geom == GEOM_CONE ? launch_geom<GEOM_CONE>(L, st) : launch_geom<GEOM_PARALLEL>(L, st);
+  if (L.P.model == MODEL_TABLE)
+    return L.P.geom == GEOM_CONE ? launch_geom<GEOM_CONE, MODEL_TABLE>(L, st)
+                                 : launch_geom<GEOM_PARALLEL, MODEL_TABLE>(L, st);
+  return L.P.geom == GEOM_CONE ? launch_geom<GEOM_CONE, MODEL_CUBIC>(L, st)
+                               : launch_geom<GEOM_PARALLEL, MODEL_CUBIC>(L, st);
 }
 
 }  // namespace trtt

@@ -1,5 +1,4 @@
-// proj3d_sweep.cu -- direct 3D projection of column-factorised views,
-// closed-form model: launches of the sweep item (sweep3d.cuh) over (view or
+// proj3d_sweep.cu -- direct 3D projection of column-factorised views: launches of the sweep item (sweep3d.cuh) over (view or
 // view group, band of detector rows, u tile), the image lines of a tile shared
 // by a cluster of CTAs where there are too few tiles for the SMs.
 //
@@ -30,7 +29,7 @@ namespace {
 
 constexpr int kMaxSplit = 8;    // portable cluster size
 
-template <int GEOM, int G, int Q, int H, int WARPS, int MINB>
+template <int GEOM, int G, int Q, int H, int WARPS, int MINB, int MODEL>
 __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const SweepLaunch A)
 {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -38,7 +37,7 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const SweepLau
   __shared__ int s_next;
   const Params3D &P = A.P;
   constexpr int US = 64 * Q;  // floats of a band row
-  constexpr size_t WB = sweep_warp_bytes<G, Q, H>();
+  constexpr size_t WB = sweep_warp_bytes<G, Q, H, MODEL>();
   const int warp = threadIdx.x >> 5;
   const int R = A.band_rows, U = A.utile, S = A.split;
   const int tile = blockIdx.x / S, rank = blockIdx.x - tile * S;
@@ -46,12 +45,19 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const SweepLau
   const int v0 = A.b.v0 + bnd * R, v1 = min(v0 + R, A.b.v1), u0 = A.b.u0 + ut * U, u1 = min(u0 + U, A.b.u1);
   constexpr int NC = 32 / H;
   const int rows = sweep_groups(R) * kSweepRows;
-  float *band = reinterpret_cast<float *>(smem);
-  unsigned char *mine = smem + sizeof(float) * (size_t)rows * US + warp * WB;
-  SweepCol *recs = reinterpret_cast<SweepCol *>(mine);
-  float2 *wtab = reinterpret_cast<float2 *>(mine + 32 * sizeof(SweepCol));
+  using Rec = typename SweepRec<MODEL>::T;
+  TableSh T{};
+  unsigned char *base = smem;
+  if constexpr (MODEL == MODEL_TABLE) {
+    table_load(P, reinterpret_cast<double *>(smem), T);
+    base += table_bytes(P);
+  }
+  float *band = reinterpret_cast<float *>(base);
+  unsigned char *mine = base + sizeof(float) * (size_t)rows * US + warp * WB;
+  Rec *recs = reinterpret_cast<Rec *>(mine);
+  float2 *wtab = reinterpret_cast<float2 *>(mine + SweepRec<MODEL>::batch * sizeof(Rec));
   float *prof = reinterpret_cast<float *>(wtab + kSweepRows * kSweepGroups * NC);
-  int *locks = reinterpret_cast<int *>(smem + sizeof(float) * (size_t)rows * US + WARPS * WB);
+  int *locks = reinterpret_cast<int *>(base + sizeof(float) * (size_t)rows * US + WARPS * WB);
   if (threadIdx.x < (int)(sizeof(View3D) / 8))
     reinterpret_cast<double *>(&sV)[threadIdx.x] =
         reinterpret_cast<const double *>(A.views + (A.groups ? A.groups[4 * blockIdx.y] : (int)blockIdx.y))[threadIdx.x];
@@ -60,8 +66,8 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const SweepLau
   for (int t = threadIdx.x; t < sweep_groups(R) * SweepStrip<Q, H>::NS; t += blockDim.x) locks[t] = 0;
   for (int t = threadIdx.x & 31; t < NC * (US + G * kSweepGuard) + G * kSweepGuard; t += 32) prof[t] = 0.f;
   __syncthreads();
-  sweep_item<GEOM, G, Q, H>(P, sV, A.vol, A.gate_stride, v0, v1, u0, u1, band, prof, recs, wtab, locks, &s_next, rank, S,
-                          A.err);
+  sweep_item<GEOM, G, Q, H, MODEL>(P, sV, A.vol, A.gate_stride, v0, v1, u0, u1, band, prof, recs, wtab, locks, &s_next,
+                                   rank, S, T, A.err);
   const int nrow = v1 - v0, ncell = u1 - u0;
   cg::cluster_group cl = cg::this_cluster();
   if (S == 1) __syncthreads(); else cl.sync();
@@ -82,7 +88,7 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const SweepLau
   if (S > 1) cl.sync();  // no CTA leaves while another reads its band
 }
 
-template <int GEOM, int G, int Q, int H, int WARPS, int MINB>
+template <int GEOM, int G, int Q, int H, int WARPS, int MINB, int MODEL = MODEL_CUBIC>
 cudaError_t launch(SweepLaunch L, cudaStream_t st)
 {
   const long slots = MINB * 148;
@@ -90,9 +96,9 @@ cudaError_t launch(SweepLaunch L, cudaStream_t st)
   L.usplit = (nu + 64 * Q / G - 1) / (64 * Q / G);
   L.utile = (nu + L.usplit - 1) / L.usplit;
   // rows per band: what the CTAs of an SM have room for; bands of one height
-  const size_t room = (227 * 1024) / MINB - 1024;
+  const size_t tab = table_bytes(L.P), room = (227 * 1024) / MINB - 1024 - tab;
   int nb = 1, R = nv;
-  while (R > 96 || sweep_smem<G, Q, H>(R, WARPS) > room) {
+  while (R > 96 || sweep_smem<G, Q, H, MODEL>(R, WARPS) > room) {
     ++nb;
     R = (nv + nb - 1) / nb;
   }
@@ -118,8 +124,8 @@ cudaError_t launch(SweepLaunch L, cudaStream_t st)
       L.split = s;
     }
   }
-  const size_t smem = sweep_smem<G, Q, H>(R, WARPS);
-  auto kern = k_fwd3d_sweep<GEOM, G, Q, H, WARPS, MINB>;
+  const size_t smem = tab + sweep_smem<G, Q, H, MODEL>(R, WARPS);
+  auto kern = k_fwd3d_sweep<GEOM, G, Q, H, WARPS, MINB, MODEL>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -153,6 +159,15 @@ cudaError_t launch_geom(const SweepLaunch &L, int G, cudaStream_t st)
   const int tiles = (nu + 255) / 256;
   int q = ((nu + tiles - 1) / tiles + 63) / 64;
   while (q > 1 && (long)((nu + 64 * q - 1) / (64 * q)) * ((nv + 63) / 64) * L.count * kMaxSplit < 2 * 148) --q;
+  if (L.P.model == MODEL_TABLE) {
+    // one CTA per SM: each holds the table (40 KB for the cubic's 10001 entries)
+    switch (q) {
+      case 1: return launch<GEOM, 1, 1, 8, 16, 1, MODEL_TABLE>(L, st);
+      case 2: return launch<GEOM, 1, 2, 8, 16, 1, MODEL_TABLE>(L, st);
+      case 3: return launch<GEOM, 1, 3, 8, 16, 1, MODEL_TABLE>(L, st);
+      default: return launch<GEOM, 1, 4, 8, 16, 1, MODEL_TABLE>(L, st);
+    }
+  }
   switch (q) {
     case 1: return launch<GEOM, 1, 1, 8, 8, 4>(L, st);
     case 2: return launch<GEOM, 1, 2, 8, 8, 3>(L, st);

@@ -1,5 +1,5 @@
-// sweep3d.cuh -- direct projection of column-factorised views, closed-form
-// model: the band of detector cells [v0, v1) x [u0, u1) of G views related by
+// sweep3d.cuh -- direct projection of column-factorised views (closed-form
+// footprint; tabulated footprint with the walks of table3d.cuh): the band of detector cells [v0, v1) x [u0, u1) of G views related by
 // turns of the grid (find_view_groups, host3d.h; G = 1: one view), accumulated
 // in shared memory, the members' values of a cell side by side.  The footprints
 // are those of the first view; member m sees there the columns turned back by
@@ -23,6 +23,7 @@
 #pragma once
 
 #include "fast3d_items.cuh"
+#include "table3d.cuh"
 
 namespace trtt {
 
@@ -149,18 +150,26 @@ template <int Q, int H> struct SweepStrip {
 };
 
 // Shared memory of one CTA: the band (rows rounded up to whole lock groups),
-// one lock per group and strip, and per warp the records of 32 columns, a table
+// one lock per group and strip, and per warp the records of a batch of columns, a table
 // of row weights and NC profile rows with guards around them.
-template <int G, int Q, int H> __host__ __device__ constexpr size_t sweep_warp_bytes()
+template <int MODEL> struct SweepRec {
+  using T = SweepCol;
+  static constexpr int batch = 32;  // columns whose records are built together
+};
+template <> struct SweepRec<MODEL_TABLE> {
+  using T = TableCol;
+  static constexpr int batch = 16;
+};
+template <int G, int Q, int H, int MODEL> __host__ __device__ constexpr size_t sweep_warp_bytes()
 {
   constexpr int NC = 32 / H;
-  return 32 * sizeof(SweepCol) + sizeof(float2) * kSweepRows * kSweepGroups * NC +
+  return SweepRec<MODEL>::batch * sizeof(typename SweepRec<MODEL>::T) + sizeof(float2) * kSweepRows * kSweepGroups * NC +
          sizeof(float) * (size_t)(NC * (64 * Q + G * kSweepGuard) + G * kSweepGuard);
 }
 __host__ __device__ constexpr int sweep_groups(int R) { return (R + kSweepRows - 1) / kSweepRows; }
-template <int G, int Q, int H> __host__ __device__ constexpr size_t sweep_smem(int R, int warps)
+template <int G, int Q, int H, int MODEL> __host__ __device__ constexpr size_t sweep_smem(int R, int warps)
 {
-  return sizeof(float) * (size_t)sweep_groups(R) * kSweepRows * 64 * Q + warps * sweep_warp_bytes<G, Q, H>() +
+  return sizeof(float) * (size_t)sweep_groups(R) * kSweepRows * 64 * Q + warps * sweep_warp_bytes<G, Q, H, MODEL>() +
          sizeof(int) * (size_t)sweep_groups(R) * SweepStrip<Q, H>::NS;
 }
 
@@ -197,6 +206,22 @@ __device__ __forceinline__ void sweep_fma(float4 &v, float wa, float wc, const f
   v.w = fmaf(wc, xc[3], fmaf(wa, xa[3], v.w));
 }
 
+// Voxels [k0, k1) of a column uc = A + B k whose footprints (half support hsm)
+// may meet cells [u0, u1).
+__device__ __forceinline__ void tile_voxels(double A, double B, double hsm, int nz, int u0, int u1, int &k0, int &k1)
+{
+  const double lo_u = (double)u0 - 1.0 - hsm, hi_u = (double)u1 + 1.0 + hsm;
+  k0 = 0;
+  k1 = nz;
+  if (fabs(B) > 1e-300) {
+    const double ka = (lo_u - A) / B, kb = (hi_u - A) / B;
+    k0 = (int)fmin(fmax(floor(fmin(ka, kb)), 0.0), (double)nz);
+    k1 = (int)fmin(fmax(ceil(fmax(ka, kb)) + 1.0, 0.0), (double)nz);
+  } else if (!(A > lo_u && A < hi_u)) {
+    k1 = 0;
+  }
+}
+
 // Record of column `a` of line `ln` into `r`; false: it misses the band or the tile.
 template <int GEOM>
 __device__ __forceinline__ bool sweep_record(const Params3D &P, const View3D &V, int i, int j, int v0, int v1, int u0,
@@ -218,16 +243,8 @@ __device__ __forceinline__ bool sweep_record(const Params3D &P, const View3D &V,
   } else {
     hsm = V.p_hs_u;
   }
-  // voxels whose footprints may meet the tile
-  const double lo_u = (double)u0 - 1.0 - hsm, hi_u = (double)u1 + 1.0 + hsm;
-  int k0 = 0, k1 = nz;
-  if (fabs(c.B) > 1e-300) {
-    const double ka = (lo_u - c.A) / c.B, kb = (hi_u - c.A) / c.B;
-    k0 = (int)fmin(fmax(floor(fmin(ka, kb)), 0.0), (double)nz);
-    k1 = (int)fmin(fmax(ceil(fmax(ka, kb)) + 1.0, 0.0), (double)nz);
-  } else if (!(c.A > lo_u && c.A < hi_u)) {
-    k1 = 0;
-  }
+  int k0, k1;
+  tile_voxels(c.A, c.B, hsm, nz, u0, u1, k0, k1);
   if (k0 >= k1) return false;
   const double ue = fma(c.B, (double)nz, c.A);
   const bool fixed = fabs(c.A) < 1e9 && fabs(ue) < 1e9 && hsm < 1e6 && sp > 0.03;
@@ -320,16 +337,111 @@ __device__ __noinline__ void sweep_profile_any(const Params3D &P, const View3D &
   }
 }
 
+// The same of the tabulated footprint.
+template <int GEOM>
+__device__ __forceinline__ bool sweep_record(const Params3D &P, const View3D &V, int i, int j, int v0, int v1, int u0,
+                                             int u1, TableCol &r, int *__restrict__ err)
+{
+  double A, B, hsm, sp;
+  if (!table_column<GEOM>(P, V, i, j, r, A, B, hsm, sp, err)) return false;
+  if (r.lo + r.n <= v0 || r.lo >= v1) return false;
+  tile_voxels(A, B, hsm, P.nz, u0, u1, r.k0, r.k1);
+  // neighbouring lanes at least two cells apart (0.2% for the rounding of the cells)
+  r.q_lanes = sp > 0.03 ? (int)ceil(2.004 / sp) : 0;
+  return r.k0 < r.k1;
+}
+
+// Voxel k of column `col` of a (gated) view.
+__device__ __forceinline__ float gate_value(const View3D &V, const float *colp, long dgate, bool gated, int k)
+{
+  float x = __ldg(colp + k);
+  if (gated) x = V.w1 != 0.f ? fmaf(V.w0, x, V.w1 * __ldg(colp + dgate + k)) : V.w0 * x;
+  return x;
+}
+
+// Profiles of a warp's columns, tabulated footprint: H lanes per column, each
+// one voxel per pass, neighbouring lanes at least two cells apart, so that a
+// step of two cells writes distinct cells.  row: the column's profile row; returns the lanes that
+// had voxels to add.
+template <int GEOM, int H>
+__device__ __forceinline__ unsigned table_profiles(const Params3D &P, const View3D &V, const TableSh &T,
+                                                   const TableCol &r, bool mine, int q, const float *colp, long dgate,
+                                                   bool gated, int u0, int u1, float *row)
+{
+  const int lig = threadIdx.x & (H - 1);
+  const int k0 = r.k0, k1 = mine ? r.k1 : k0, nk = __reduce_max_sync(FULLM, k1 - k0);
+  unsigned touched = 0;
+#pragma unroll 1
+  for (int pp = 0, sub = 0; pp < nk;) {
+    const int k = k0 + pp + sub + q * lig;
+    if (++sub == q) {
+      sub = 0;
+      pp += H * q;
+    }
+    const float x = k < k1 ? gate_value(V, colp, dgate, gated, k) : 0.f;
+    const unsigned some = __ballot_sync(FULLM, x != 0.f);
+    if (!some) continue;
+    touched |= some;
+    TableVox v;
+    table_voxel<GEOM>(P, V, T, r, table_kc<GEOM>(V, k), u0, u1, v);
+    if (x == 0.f) v.n = 0;
+    const float xr = x * v.rho;
+    const int steps = __reduce_max_sync(FULLM, v.n > 0 ? v.s + v.n : 0);
+    float *cell = row + (v.f - u0);
+    double l = (double)(-v.l0), e0 = table_at(T, dadd(v.start, dmul(l, v.inc)));
+#pragma unroll 1
+    for (int t = 0; t < steps; t += 2) {
+      const double e1 = table_at(T, dadd(v.start, dmul(l + 1.0, v.inc)));
+      l += 2.0;
+      const double e2 = table_at(T, dadd(v.start, dmul(l, v.inc)));
+      const bool in0 = (unsigned)(t - v.s) < (unsigned)v.n, in1 = (unsigned)(t + 1 - v.s) < (unsigned)v.n;
+      float y0 = 0.f, y1 = 0.f;
+      if (in0) y0 = cell[0];
+      if (in1) y1 = cell[1];
+      y0 = fmaf((float)(e1 - e0), xr, y0);
+      y1 = fmaf((float)(e2 - e1), xr, y1);
+      if (in0) cell[0] = y0;
+      if (in1) cell[1] = y1;
+      __syncwarp();
+      e0 = e2;
+      cell += 2;
+    }
+  }
+  return touched;
+}
+
+// One column's by the whole warp with atomics: columns whose voxels nearly
+// coincide on the detector.
+template <int GEOM>
+__device__ __noinline__ void table_profile_any(const Params3D &P, const View3D &V, const TableSh &T, const TableCol &r,
+                                               const float *colp, long dgate, bool gated, int u0, int u1, float *row)
+{
+  for (int k = r.k0 + (threadIdx.x & 31); k < r.k1; k += 32) {
+    const float x = gate_value(V, colp, dgate, gated, k);
+    if (x == 0.f) continue;
+    TableVox v;
+    table_voxel<GEOM>(P, V, T, r, table_kc<GEOM>(V, k), u0, u1, v);
+    for (int t = v.s; t < v.s + v.n; ++t) {
+      const double l = (double)(t - v.l0);
+      const float w = (float)(table_at(T, dadd(v.start, dmul(l + 1.0, v.inc))) -
+                              table_at(T, dadd(v.start, dmul(l, v.inc))));
+      atomicAdd(row + (v.f - u0) + t, w * (x * v.rho));
+    }
+  }
+}
+
 // All threads of the CTA call it; band, prof (this warp's profile rows) and
 // locks are zero on entry, prof zero on exit; no final barrier.  `next`: the
 // CTA's line counter (0 on entry); the CTA takes lines rank, rank + split, ...
 // The tile has u1 - u0 <= 64 Q / G cells.
-template <int GEOM, int G, int Q, int H>
+template <int GEOM, int G, int Q, int H, int MODEL>
 __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, const float *__restrict__ vol,
                                            long gate_stride, int v0, int v1, int u0, int u1, float *band, float *prof,
-                                           SweepCol *recs, float2 *wtab, int *locks, int *next, int rank, int split,
-                                           int *__restrict__ err)
+                                           typename SweepRec<MODEL>::T *recs, float2 *wtab, int *locks, int *next,
+                                           int rank, int split, const TableSh &T, int *__restrict__ err)
 {
+  using Rec = typename SweepRec<MODEL>::T;
+  constexpr int RB = SweepRec<MODEL>::batch;
   using VecG = typename SweepVec<G>::T;
   using Strip = SweepStrip<Q, H>;
   constexpr int NC = Strip::NC, SP = Strip::SP, NS = Strip::NS;
@@ -357,11 +469,11 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
       a0 += seg * len;
       a1 = min(a1, a0 + len);
     }
-    for (int ab = a0; ab < a1; ab += 32) {
-      // ---- records of up to 32 columns, without gaps ---------------------
+    for (int ab = a0; ab < a1; ab += RB) {
+      // ---- records of up to RB columns, without gaps ---------------------
       const int a = ab + lane;
-      SweepCol rec;
-      const bool hit = a < a1 &&
+      Rec rec;
+      const bool hit = a < a1 && (RB == 32 || lane < RB) &&
                        sweep_record<GEOM>(P, V, S.axis ? ln : a, S.axis ? a : ln, v0, v1, u0, u1, rec, err);
       rec.col = a;
       const unsigned mask = __ballot_sync(FULLM, hit);
@@ -372,12 +484,25 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
       for (int b = 0; b < cnt; b += NC) {
         // ---- profiles of columns b .. b + NC - 1 -------------------------
         const bool mine = b + grp < cnt;
-        const SweepCol &r = recs[mine ? b + grp : b];
-        const int p0 = r.p0, p1 = mine ? r.p1 : p0;
-        int q = r.q;
+        const Rec &r = recs[mine ? b + grp : b];
         unsigned touched = 0;
-        if (!__any_sync(FULLM, q == 0)) {
-          q = __reduce_max_sync(FULLM, q);
+        if constexpr (MODEL == MODEL_TABLE) {
+          if (!__any_sync(FULLM, r.q_lanes == 0)) {
+            const float *colp = volg + turned_col(S.axis ? ln : r.col, S.axis ? r.col : ln, 0, nx, ny) * nz;
+            touched = table_profiles<GEOM, H>(P, V, T, r, mine, __reduce_max_sync(FULLM, r.q_lanes), colp, dgate,
+                                              gated, u0, u1, prof + kSweepGuard + grp * PS);
+          } else {
+            for (int g = 0; g < NC && b + g < cnt; ++g) {
+              const Rec &o = recs[b + g];
+              const float *colp = volg + turned_col(S.axis ? ln : o.col, S.axis ? o.col : ln, 0, nx, ny) * nz;
+              table_profile_any<GEOM>(P, V, T, o, colp, dgate, gated, u0, u1, prof + kSweepGuard + g * PS);
+            }
+            touched = FULLM;
+            __syncwarp();
+          }
+        } else if (!__any_sync(FULLM, r.q == 0)) {
+          const int p0 = r.p0, p1 = mine ? r.p1 : p0;
+          const int q = __reduce_max_sync(FULLM, r.q);
           const int steps = __reduce_max_sync(FULLM, r.steps), np = __reduce_max_sync(FULLM, p1 - p0);
           const int ci = S.axis ? ln : r.col, cj = S.axis ? r.col : ln;
           const float *colp[G];
@@ -474,7 +599,7 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
           }
         } else {
           for (int g = 0; g < NC && b + g < cnt; ++g) {
-            const SweepCol &o = recs[b + g];
+            const Rec &o = recs[b + g];
             sweep_profile_any<GEOM, G>(P, V, vol, gate_stride, S.axis ? ln : o.col, S.axis ? o.col : ln, o.p0, o.p1,
                                     u0, ncell, prof + G * (kSweepGuard + g * PS));
           }
@@ -495,14 +620,18 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
           // table of weights [row][column], rows of lock groups gb .. gb + ng
           for (int e = lane; e < ng * kSweepRows * NC; e += 32) {
             const int g = e % NC;
-            const SweepCol &o = recs[min(b + g, cnt - 1)];
+            const Rec &o = recs[min(b + g, cnt - 1)];
             const int l = v0 + gb * kSweepRows + e / NC - o.lo;
             float w = 0.f;
             if (((live >> (g * H)) & 1u) && l >= 0 && l < o.n) {
-              AxisCubic ax;
-              ax.start = o.vstart;
-              ax.inc = o.vinc;
-              w = edge_cubic(ax, l + 1) - edge_cubic(ax, l);
+              if constexpr (MODEL == MODEL_TABLE) {
+                w = table_weight_v(T, o, l);
+              } else {
+                AxisCubic ax;
+                ax.start = o.vstart;
+                ax.inc = o.vinc;
+                w = edge_cubic(ax, l + 1) - edge_cubic(ax, l);
+              }
             }
             wtab[e] = f2(w);
           }

@@ -50,6 +50,7 @@ struct Params3D {
   double step;       // step_footprint
   double coord0;     // coord_footprint[0]
   int size;          // size_footprint
+  int tab0, tab1;    // the table is constant up to slot tab0 and from slot tab1 on
   int pad_;
 };
 
