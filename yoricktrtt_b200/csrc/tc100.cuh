@@ -34,6 +34,20 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
   return d;
 }
 
+// K-major rows of `row` bytes (32, 64 or 128) in the swizzle of that width (TMA's
+// pattern: address bits 4.. xor bits 7.., taken from the address itself, so a
+// matrix may start at any row of a buffer aligned to the pattern): stride byte
+// offset 8 rows, layout 6, 4, 2.
+__device__ __forceinline__ uint64_t sdesc_swz(uint32_t saddr, uint32_t row)
+{
+  uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(((8u * row) >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)(row == 32u ? 6u : row == 64u ? 4u : 2u) << 61;
+  return d;
+}
+
 // Instruction descriptor, kind::f16 with BF16 A and B and FP32 D:
 //   bits 4-5 D format (1 = F32), 7-9 A format (1 = BF16), 10-12 B format,
 //   bit 15 A major (0 = K, 1 = MN), bit 16 B major, 17-22 N >> 3, 24-28 M >> 4.
@@ -57,6 +71,38 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
       :
       : "r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z),
         "r"(z)
+      : "memory");
+}
+
+// The same, and the commit, called by a whole warp whose arguments are the same
+// in every lane: one elected lane issues.  The operands then stay in uniform
+// registers; from a single thread's branch each is moved there first.  The
+// descriptors come as low and high words: only the low one differs between MMAs.
+__device__ __forceinline__ void mma_bf16_warp(uint32_t d_tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                              uint32_t idesc, uint32_t accumulate)
+{
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, e;\n\t"
+      ".reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %2};\n\t"
+      "mov.b64 b, {%3, %4};\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t"
+      "}\n"
+      :
+      : "r"(d_tmem), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void mma_commit_warp(uint64_t *mbar)
+{
+  asm volatile(
+      "{\n\t"
+      ".reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(smem_addr(mbar))
       : "memory");
 }
 
@@ -109,6 +155,34 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
                : "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Three such loads in flight together.
+__device__ __forceinline__ void tmem_ld16x3(uint32_t t0, uint32_t t1, uint32_t t2, float (&v)[3][16])
+{
+  uint32_t r[3][16];
+  const uint32_t at[3] = {t0, t1, t2};
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[k][0]), "=r"(r[k][1]), "=r"(r[k][2]), "=r"(r[k][3]), "=r"(r[k][4]), "=r"(r[k][5]),
+          "=r"(r[k][6]), "=r"(r[k][7]), "=r"(r[k][8]), "=r"(r[k][9]), "=r"(r[k][10]), "=r"(r[k][11]),
+          "=r"(r[k][12]), "=r"(r[k][13]), "=r"(r[k][14]), "=r"(r[k][15])
+        : "r"(at[k])
+        : "memory");
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[k][0]), "+r"(r[k][1]), "+r"(r[k][2]), "+r"(r[k][3]), "+r"(r[k][4]), "+r"(r[k][5]),
+                   "+r"(r[k][6]), "+r"(r[k][7]), "+r"(r[k][8]), "+r"(r[k][9]), "+r"(r[k][10]), "+r"(r[k][11]),
+                   "+r"(r[k][12]), "+r"(r[k][13]), "+r"(r[k][14]), "+r"(r[k][15])
+                 :
+                 : "memory");
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[k][i] = __uint_as_float(r[k][i]);
 }
 
 // mbarriers --------------------------------------------------------------

@@ -114,6 +114,62 @@ struct FwdArgs {
   uint32_t tmem_cols;
 };
 
+// Output channels [j, j + 16) of row p: bias, activation and the output layout
+// of the mode.
+__device__ __forceinline__ void fwd_emit(const FwdArgs &a, long p, int j, float (&v)[16])
+{
+  const int n = a.n;
+        if (a.bias && a.mode != kFwdGrad) {
+  #pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] += a.bias[j + i];
+        }
+        if (a.mode == kFwdAct) {
+          uint4 q0, q1;
+          q0.x = pack_bf16x2(act(v[0], a.slope), act(v[1], a.slope));
+          q0.y = pack_bf16x2(act(v[2], a.slope), act(v[3], a.slope));
+          q0.z = pack_bf16x2(act(v[4], a.slope), act(v[5], a.slope));
+          q0.w = pack_bf16x2(act(v[6], a.slope), act(v[7], a.slope));
+          q1.x = pack_bf16x2(act(v[8], a.slope), act(v[9], a.slope));
+          q1.y = pack_bf16x2(act(v[10], a.slope), act(v[11], a.slope));
+          q1.z = pack_bf16x2(act(v[12], a.slope), act(v[13], a.slope));
+          q1.w = pack_bf16x2(act(v[14], a.slope), act(v[15], a.slope));
+          uint4 *dst = reinterpret_cast<uint4 *>(static_cast<bf16 *>(a.y) + p * n + j);
+          dst[0] = q0;
+          dst[1] = q1;
+        } else if (a.mode == kFwdF32) {
+          float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(a.y) + p * n + j);
+  #pragma unroll
+          for (int i = 0; i < 4; ++i)
+            dst[i] = make_float4(act(v[4 * i], a.slope), act(v[4 * i + 1], a.slope),
+                                 act(v[4 * i + 2], a.slope), act(v[4 * i + 3], a.slope));
+        } else if (a.mode == kFwdHead) {
+          if (j == 0) static_cast<float *>(a.y)[p] = a.resid[p] + v[0];
+        } else {  // kFwdGrad
+          bf16 *base;
+          int ld, c0;
+          if (j < a.n1) { base = static_cast<bf16 *>(a.y); ld = a.n1; c0 = j; }
+          else { base = static_cast<bf16 *>(a.y2); ld = n - a.n1; c0 = j - a.n1; }
+          uint4 *dst = reinterpret_cast<uint4 *>(base + p * ld + c0);
+          if (a.accumulate) {
+            const uint4 o0 = dst[0], o1 = dst[1];
+            const uint32_t ow[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+  #pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float2 f = unpack_bf16x2(ow[i]);
+              v[2 * i] += f.x;
+              v[2 * i + 1] += f.y;
+            }
+          }
+          uint4 q0, q1;
+          q0.x = pack_bf16x2(v[0], v[1]); q0.y = pack_bf16x2(v[2], v[3]);
+          q0.z = pack_bf16x2(v[4], v[5]); q0.w = pack_bf16x2(v[6], v[7]);
+          q1.x = pack_bf16x2(v[8], v[9]); q1.y = pack_bf16x2(v[10], v[11]);
+          q1.z = pack_bf16x2(v[12], v[13]); q1.w = pack_bf16x2(v[14], v[15]);
+          dst[0] = q0;
+          dst[1] = q1;
+        }
+}
+
 // Epilogue of the forward / input-gradient convolution: the S accumulators
 // of 128 rows x n columns in tensor memory (warp w reads TMEM lanes
 // 32w..32w+31) to bias, activation and the output layout of the mode.
@@ -129,56 +185,7 @@ __device__ __forceinline__ void fwd_epilogue(const FwdArgs &a, uint32_t tmem, lo
     for (int j = 0; j < n; j += 16) {
       float v[16];
       tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(s * n + j), v);
-      if (!inside) continue;
-      if (a.bias && a.mode != kFwdGrad) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] += a.bias[j + i];
-      }
-      if (a.mode == kFwdAct) {
-        uint4 q0, q1;
-        q0.x = pack_bf16x2(act(v[0], a.slope), act(v[1], a.slope));
-        q0.y = pack_bf16x2(act(v[2], a.slope), act(v[3], a.slope));
-        q0.z = pack_bf16x2(act(v[4], a.slope), act(v[5], a.slope));
-        q0.w = pack_bf16x2(act(v[6], a.slope), act(v[7], a.slope));
-        q1.x = pack_bf16x2(act(v[8], a.slope), act(v[9], a.slope));
-        q1.y = pack_bf16x2(act(v[10], a.slope), act(v[11], a.slope));
-        q1.z = pack_bf16x2(act(v[12], a.slope), act(v[13], a.slope));
-        q1.w = pack_bf16x2(act(v[14], a.slope), act(v[15], a.slope));
-        uint4 *dst = reinterpret_cast<uint4 *>(static_cast<bf16 *>(a.y) + p * n + j);
-        dst[0] = q0;
-        dst[1] = q1;
-      } else if (a.mode == kFwdF32) {
-        float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(a.y) + p * n + j);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          dst[i] = make_float4(act(v[4 * i], a.slope), act(v[4 * i + 1], a.slope),
-                               act(v[4 * i + 2], a.slope), act(v[4 * i + 3], a.slope));
-      } else if (a.mode == kFwdHead) {
-        if (j == 0) static_cast<float *>(a.y)[p] = a.resid[p] + v[0];
-      } else {  // kFwdGrad
-        bf16 *base;
-        int ld, c0;
-        if (j < a.n1) { base = static_cast<bf16 *>(a.y); ld = a.n1; c0 = j; }
-        else { base = static_cast<bf16 *>(a.y2); ld = n - a.n1; c0 = j - a.n1; }
-        uint4 *dst = reinterpret_cast<uint4 *>(base + p * ld + c0);
-        if (a.accumulate) {
-          const uint4 o0 = dst[0], o1 = dst[1];
-          const uint32_t ow[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float2 f = unpack_bf16x2(ow[i]);
-            v[2 * i] += f.x;
-            v[2 * i + 1] += f.y;
-          }
-        }
-        uint4 q0, q1;
-        q0.x = pack_bf16x2(v[0], v[1]); q0.y = pack_bf16x2(v[2], v[3]);
-        q0.z = pack_bf16x2(v[4], v[5]); q0.w = pack_bf16x2(v[6], v[7]);
-        q1.x = pack_bf16x2(v[8], v[9]); q1.y = pack_bf16x2(v[10], v[11]);
-        q1.z = pack_bf16x2(v[12], v[13]); q1.w = pack_bf16x2(v[14], v[15]);
-        dst[0] = q0;
-        dst[1] = q1;
-      }
+      if (inside) fwd_emit(a, p, j, v);
     }
   }
 }
@@ -567,6 +574,290 @@ __global__ void __launch_bounds__(192) k_conv3_fwd_pers(const FwdArgs a, const _
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, a.tmem_cols);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// forward / input-gradient convolution, input planes streamed along z
+// ---------------------------------------------------------------------------
+// A CTA takes 128 S rows of the padded plane (m0 .. m0 + 128 S - 1; output rows
+// are all but the first and the last) over a segment [za, zb) of output planes
+// and streams the input planes past them.  Input plane z feeds the outputs
+// z - 1, z and z + 1, which accumulate side by side in tensor memory (buffer
+// zo % NB), so a row is staged once, not once per dz.  The three dx taps are
+// fused into the N dimension: for each (dz, dy) one MMA of 128 x 3n x 16
+// computes D_dx[r] = X[r + dz, dy] W_dx, and the epilogue adds the neighbouring
+// rows, out[r] = D_0[r-1] + D_1[r] + D_2[r+1] (rows are tensor-memory lanes:
+// shuffles, and the rows at a warp's edge through shared memory): 9 MMAs per 16
+// channels and 128 rows, not 27.  All weights stay in shared memory.
+//   4 S HW warps: epilogue, warp (s, q, j): 32 rows 128 s + 32 q, channels
+//     [j, j + 16): it takes its three blocks to registers, which frees the
+//     buffer, and then exchanges rows and writes;
+//   warp EW, one thread: producer, stages (input plane, 16 to 64 channels) into
+//     the ring by TMA, a row's channels as 32, 64 or 128 bytes in the swizzle of
+//     that width.  Boxes of 8 channels would write 16 bytes of shared memory per
+//     cycle and fetch each 32-byte sector twice (120 us of the first layer below
+//     by themselves);
+//   S warps: MMA issuers of one sub-tile each (an MMA takes a warp about 60
+//     cycles to issue, the tensor core about 45).  Per stage dz = 2, 1, 0; the
+//     plane's last stage completes output z - 1 (`accf`), the first dz = 0 of a
+//     plane waits for the epilogue that had the buffer before (`acce`).
+// Input planes 0 and d + 1 are zero and left out.  Waits and the way out after a
+// failed one: as k_conv3_fwd_pers (the epilogue warps meet on bounded mbarriers,
+// never on a block barrier).
+//
+// Measured against k_conv3_fwd_pers: 48 -> 16 channels at 128^3 269 -> 127 us, 32
+// -> 32 at 2 x 64^3 66 -> 54 us.  Bounds: the first 100 us of MMAs (A from shared
+// memory: 4 KB each for 3n columns), staging 54 us beside them; the second the
+// chain of waits per plane (23 us without any load or MMA) and 41 us of MMAs.
+struct ZArgs {
+  int S, tiles, segs, len;    // sub-tiles; tiles per plane, z segments per volume and their length
+  int hw;                     // epilogue warps per 32 rows, n / 16
+  int w_bytes, edge_bytes;    // weights and edge rows ahead of the ring
+};
+
+constexpr int kZStages = 12;
+
+__host__ __device__ constexpr int z_threads(int S, int HW) { return 128 * S * HW + 32 + 32 * S; }
+// Channels per row of a stage: 32, 64 or 128 bytes, the swizzle's widths.
+__host__ __device__ inline int z_channels(int c) { return c % 64 == 0 ? 64 : c % 32 == 0 ? 32 : 16; }
+
+// Position in the ring: buffer and the parity of its use (no divisions).
+struct RingPos {
+  int slot = 0;
+  uint32_t par = 0;
+  __device__ __forceinline__ void next(int nstg, int by = 1)
+  {
+    slot += by;
+    if (slot >= nstg) {
+      slot -= nstg;
+      par ^= 1u;
+    }
+  }
+};
+
+template <int S, int HW, int NB>
+__global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdArgs a, const ZArgs z, const __grid_constant__ FwdMaps maps)
+{
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[kZStages], empty[kZStages], accf[NB], acce[NB], edgeb, finb;
+  __shared__ uint32_t s_taddr;
+  __shared__ volatile int s_bad;
+  __shared__ int s_issued, s_consumed;
+  constexpr int EW = 4 * S * HW;  // epilogue warps; then the producer and S issuers
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int G = a.groups, n = a.n, nstg = a.nstg, wp = a.g.wp;
+  const uint32_t sbase = tc::smem_addr(smem), ring = sbase + (uint32_t)(z.w_bytes + z.edge_bytes);
+  float *edge = reinterpret_cast<float *>(smem + z.w_bytes);  // [2][4 S + 2][2][n]
+  const int unit = blockIdx.x, seg = unit % z.segs, tile = (unit / z.segs) % z.tiles, vol = unit / (z.segs * z.tiles);
+  const int za = 1 + seg * z.len, zb = min(za + z.len, a.g.d + 1);
+  const int zlo = max(za - 1, 1), zhi = min(zb, a.g.d);  // input planes
+  const int m0 = wp + tile * (128 * S - 2) - 1;           // in-plane row of tensor-memory lane 0
+  const long vrow = (long)vol * a.g.vol;
+
+  if (tid == 0) {
+    for (int i = 0; i < nstg; ++i) {
+      tc::mbar_init(&full[i], 1);
+      tc::mbar_init(&empty[i], S);
+    }
+    for (int b = 0; b < NB; ++b) {
+      tc::mbar_init(&accf[b], S);
+      tc::mbar_init(&acce[b], EW);
+    }
+    tc::mbar_init(&edgeb, EW);
+    tc::mbar_init(&finb, S);
+    s_bad = 0;
+    s_issued = 0;
+    s_consumed = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == EW + 1) tc::tmem_alloc(&s_taddr, a.tmem_cols);
+  // weights: [dz][g][dy][chunk][dx n + co][8] from [dz G + g][dy 3 + dx][chunk][co][8]
+  for (int e = tid; e < 27 * G * 2 * n; e += blockDim.x) {
+    const int co = e % n, c = (e / n) & 1, t9 = (e / (2 * n)) % 9, st = e / (18 * n);
+    const int dy = t9 / 3, dx = t9 - 3 * dy;
+    reinterpret_cast<uint4 *>(smem)[((st * 3 + dy) * 2 + c) * 3 * n + dx * n + co] =
+        __ldg(reinterpret_cast<const uint4 *>(a.wpack) + e);
+  }
+  tc::fence_async_smem();
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = s_taddr;
+  const uint32_t cols = (uint32_t)(3 * n);
+
+  if (warp == EW) {
+    if (lane == 0) {
+      // producer
+      RingPos p;
+      int c = 0;
+      for (int zi = zlo; zi <= zhi && !s_bad; ++zi) {
+        const int hb = (int)(vrow + (long)zi * a.g.plane) + m0 - wp;
+        for (int ch = 0; ch < a.c1 + a.c2;) {
+          const bool first = ch < a.c1;
+          const int ic = z_channels(first ? a.c1 : a.c2), x = first ? ch : ch - a.c1;
+          if (c >= nstg && !tc::mbar_wait(&empty[p.slot], p.par ^ 1u, kWaitNs)) s_bad = 1;
+          if (s_bad) break;
+          const CUtensorMap *mfull = first ? &maps.x1_full : &maps.x2_full;
+          const CUtensorMap *mtail = first ? &maps.x1_tail : &maps.x2_tail;
+          const uint32_t hs = ring + (uint32_t)(p.slot * a.stage_bytes);
+          tc::mbar_arrive_expect_tx(&full[p.slot], (uint32_t)(a.rh * ic * 2));
+          for (int r0 = 0; r0 < a.rh; r0 += 256)
+            tc::tma_load_2d(hs + (uint32_t)(r0 * ic * 2), a.rh - r0 >= 256 ? mfull : mtail, x, hb + r0, &full[p.slot]);
+          ++c;
+          p.next(nstg);
+          ch += ic;
+        }
+      }
+      s_issued = c;
+    }
+  } else if (warp >= EW + 1) {
+    // MMA issuer of sub-tile s (the whole warp, every value the same in its lanes)
+    const uint32_t idesc = tc::idesc_bf16(128, 3 * n, 0, 0);
+    const int s = warp - (EW + 1);
+    auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
+    const uint32_t bstep = uniform((uint32_t)(6 * G) * cols);
+    RingPos p;
+    int used = 0;  // stages waited for
+    bool ok = true;
+    // accumulators of zi - 1, zi, zi + 1
+    int b2 = (zlo + NB - 1) % NB, b1 = zlo % NB, b0 = (zlo + 1) % NB;
+    for (int zi = zlo; zi <= zhi && ok; ++zi) {
+      const bool v2 = zi - 1 >= za, v1 = zi >= za && zi < zb, v0 = zi + 1 < zb;
+      // output zi + 1 starts here; output 1 already with plane 1 (0 is left out)
+      const uint32_t acc[3] = {uniform(tmem + (uint32_t)(b0 * S + s) * cols), uniform(tmem + (uint32_t)(b1 * S + s) * cols),
+                               uniform(tmem + (uint32_t)(b2 * S + s) * cols)};
+      for (int ch = 0; ch < 16 * G;) {
+        const int ic = z_channels(ch < a.c1 ? a.c1 : a.c2);
+        const bool in = tc::mbar_wait(&full[p.slot], p.par, kWaitNs);
+        ok = __all_sync(0xffffffffu, in && !s_bad);  // (votes keep the loop's values uniform)
+        if (!ok) break;
+        ++used;
+        tc::fence_after_sync();
+        const uint32_t row = 2u * ic;
+        const uint64_t ad = tc::sdesc_swz(ring + (uint32_t)(p.slot * a.stage_bytes) + 128u * s * row, row);
+        const uint32_t ahi = uniform((uint32_t)(ad >> 32)), ydy = uniform((uint32_t)wp * (row >> 4));
+#pragma unroll 1
+        for (int k = 0; k < ic; k += 16) {
+          const int g = (ch + k) >> 4;
+          // descriptors count 16 bytes
+          const uint64_t bd = tc::sdesc(sbase + (uint32_t)(3 * g) * 2u * cols * 16u, cols * 16u, 128u);
+          const uint32_t alo = uniform((uint32_t)ad + (uint32_t)(k >> 3));
+          const uint32_t blo = uniform((uint32_t)bd), bhi = uniform((uint32_t)(bd >> 32));
+          auto mma = [&](int dz, int dy, uint32_t add) {
+            tc::mma_bf16_warp(acc[dz], alo + (uint32_t)dy * ydy, ahi, blo + (uint32_t)dz * bstep + (uint32_t)(2 * dy) * cols,
+                              bhi, idesc, add);
+          };
+          const bool wait = g == 0 && v0 && zi + 1 - NB >= za;
+          // MMAs of the three output planes alternate: those into one accumulator
+          // follow each other by their latency
+#pragma unroll
+          for (int dy = 0; dy < 3; ++dy) {
+            if (v2) mma(2, dy, 1u);
+            if (v1) mma(1, dy, (dy > 0 || g > 0 || zi > 1) ? 1u : 0u);
+            if (v0 && !wait) mma(0, dy, (dy > 0 || g > 0) ? 1u : 0u);
+          }
+          if (wait) {
+            // the buffer is free once the epilogue of zi + 1 - NB has read it
+            const bool free = tc::mbar_wait(&acce[b0], (uint32_t)((zi + 1 - za) / NB - 1) & 1u, kWaitNs);
+            ok = __all_sync(0xffffffffu, free);
+            if (!ok) break;
+            tc::fence_after_sync();
+#pragma unroll
+            for (int dy = 0; dy < 3; ++dy) mma(0, dy, dy > 0 ? 1u : 0u);
+          }
+        }
+        if (!ok) break;
+        ch += ic;
+        if (ch == 16 * G) {
+          if (v2) tc::mma_commit_warp(&accf[b2]);
+          if (v1 && zi == a.g.d) tc::mma_commit_warp(&accf[b1]);
+        }
+        tc::mma_commit_warp(&empty[p.slot]);
+        p.next(nstg);
+      }
+      b2 = b1;
+      b1 = b0;
+      b0 = b0 + 1 == NB ? 0 : b0 + 1;
+    }
+    if (!ok) s_bad = 1;
+    if (s == 0 && lane == 0) s_consumed = used;
+    tc::mma_commit_warp(&finb);  // arrives once every MMA issued above has completed
+  } else {
+    // epilogue
+    const int q = warp & 3, s = (warp >> 2) % S, j = 16 * ((warp >> 2) / S);
+    const int blk = 4 * s + q;  // blocks of 32 rows in order
+    const int ip = m0 + 32 * blk + lane, y = ip / wp, x = ip - y * wp, r = 32 * blk + lane;
+    const bool inside = r > 0 && r < 128 * S - 1 && y >= 1 && y <= a.g.h && x >= 1 && x <= a.g.w;
+    for (int zo = za; zo < zb; ++zo) {
+      const int u = zo - za;
+      const bool full_ok = tc::mbar_wait(&accf[zo % NB], (uint32_t)(u / NB) & 1u, kWaitNs);
+      if (!__all_sync(0xffffffffu, full_ok)) {
+        s_bad = 1;
+        break;
+      }
+      tc::fence_after_sync();
+      const uint32_t acc = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)((zo % NB) * S + s) * cols;
+      float *ed = edge + (u & 1) * (4 * S + 2) * 2 * n;
+      float v[3][16];
+      tc::tmem_ld16x3(acc + (uint32_t)j, acc + (uint32_t)(n + j), acc + (uint32_t)(2 * n + j), v);
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&acce[zo % NB]);  // the buffer is free
+      // D_0 of the block's last row and D_2 of its first, to the neighbours
+      if (lane == 31) {
+        float4 *o = reinterpret_cast<float4 *>(ed + ((blk + 2) * 2 + 0) * n + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = make_float4(v[0][4 * i], v[0][4 * i + 1], v[0][4 * i + 2], v[0][4 * i + 3]);
+      }
+      if (lane == 0) {
+        float4 *o = reinterpret_cast<float4 *>(ed + (blk * 2 + 1) * n + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = make_float4(v[2][4 * i], v[2][4 * i + 1], v[2][4 * i + 2], v[2][4 * i + 3]);
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&edgeb);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        v[0][i] = __shfl_up_sync(0xffffffffu, v[0][i], 1);
+        v[2][i] = __shfl_down_sync(0xffffffffu, v[2][i], 1);
+      }
+      const bool edge_ok = tc::mbar_wait(&edgeb, (uint32_t)u & 1u, kWaitNs);
+      if (!__all_sync(0xffffffffu, edge_ok)) {
+        s_bad = 1;
+        break;
+      }
+      if (lane == 0 || lane == 31) {  // rows before the first and after the last block stay unused
+        const float4 *o = reinterpret_cast<const float4 *>(ed + ((blk + 1) * 2 + (lane ? 1 : 0)) * n + j);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 f = o[i];
+          const float w[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (lane) v[2][4 * i + k] = w[k];
+            else v[0][4 * i + k] = w[k];
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) v[1][i] = (v[0][i] + v[1][i]) + v[2][i];
+      if (inside) fwd_emit(a, vrow + (long)zo * a.g.plane + ip, j, v[1]);
+      if (__any_sync(0xffffffffu, s_bad != 0)) break;
+    }
+  }
+  const bool fin_ok = tc::mbar_wait(&finb, 0, kWaitNs);
+  __syncthreads();
+  if (tid == 0 && (s_bad || !fin_ok)) {
+    // copies issued for stages the MMAs never consumed
+    for (int c = s_consumed; c < s_issued; ++c) tc::mbar_wait(&full[c % nstg], (uint32_t)(c / nstg) & 1u, kWaitNs);
+    atomicExch(&g_unet_err, 1);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == EW + 1) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, a.tmem_cols);
   }
@@ -1234,6 +1525,49 @@ FwdPlan fwd_plan_pers(int n, int groups, const Grid3 &g, int *S)
   return p;
 }
 
+// Layout of the z-streaming kernel; false where it does not apply: the
+// accumulators in tensor memory, all weights and two stages in shared memory.  Segments of z: fewest waves of CTAs (one per SM) times
+// planes per CTA (two input planes of halo, and about two for start and end).
+bool fwd_plan_z(int n, int c1, int c2, const Grid3 &g, FwdPlan &p, ZArgs &z)
+{
+  const int groups = (c1 + c2) / 16, ic = std::max(z_channels(c1), c2 ? z_channels(c2) : 0);
+
+  z.S = n == 16 ? 3 : 1;
+  z.hw = n / 16;
+  const int nb = n == 32 ? 5 : 3;  // accumulators
+  // 16 outputs, or 32 with two stages a plane or more and a slab of at most 3.3
+  // rows per output row.  Elsewhere the per-plane waits and the slab cost more
+  // than the fused taps save: 16 -> 32 at 96^3 62 us per tile, 87 here, 32 -> 32 at
+  // 40 x 128 x 160 99 against 101; but 32 -> 32 at 128^3 209 against 165.
+  if (n > 32 || (n == 32 && (groups < 2 || g.wp > 150)) || g.rows >= (1L << 31) - (1L << 20)) return false;
+  p.tmem_cols = pow2_cols(nb * z.S * 3 * n);
+  p.rh = 128 * z.S + 2 * g.wp;
+  p.cs = 0;
+  p.stage_bytes = ((p.rh * 2 * ic + 1023) / 1024) * 1024;
+  z.w_bytes = ((27 * groups * 16 * n * 2 + 1023) / 1024) * 1024;
+  z.edge_bytes = ((2 * (4 * z.S + 2) * 2 * n * 4 + 1023) / 1024) * 1024;
+  const int room = 224 * 1024 - z.w_bytes - z.edge_bytes;
+  p.nstg = std::min(kZStages, room / p.stage_bytes);
+  if (room <= 0 || p.nstg < 2) return false;
+  p.smem = residency_smem(z.w_bytes + z.edge_bytes + p.nstg * p.stage_bytes, p.tmem_cols);
+  if (p.smem > 226 * 1024) return false;
+  const long t = 128 * z.S - 2, tiles = ((long)g.h * g.wp + t - 1) / t;
+  if (tiles * g.nb * g.d > 0x7FFFFFFFL) return false;
+  z.tiles = (int)tiles;
+  double best = 1e300;
+  for (int len = 1; len <= g.d; ++len) {
+    const long segs = (g.d + len - 1) / len, units = tiles * g.nb * segs;
+    const double cost = (double)((units + 147) / 148) * (len + 4.0);
+    if (cost < best) {
+      best = cost;
+      z.len = len;
+      z.segs = (int)segs;
+    }
+  }
+  p.tiles = tiles * g.nb * z.segs;
+  return true;
+}
+
 // cuTensorMapEncodeTiled, reached through the runtime (no driver library
 // link); null when the driver does not provide it.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -1256,17 +1590,20 @@ EncodeTiledFn encode_tiled()
 }
 
 // Tensor map of a padded channels-last activation (rows x c BF16): boxes of
-// 8 channels x box_rows rows, zeros outside the tensor.
-bool act_map(CUtensorMap *m, const void *base, int c, long rows, int box_rows)
+// box_c channels x box_rows rows (16 to 64 channels: swizzled by the width of a
+// row), zeros outside the tensor.
+bool act_map(CUtensorMap *m, const void *base, int c, long rows, int box_rows, int box_c = 8)
 {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)c, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)c * 2};
-  const cuuint32_t box[2] = {8u, (cuuint32_t)box_rows};
+  const cuuint32_t box[2] = {(cuuint32_t)box_c, (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1u, 1u};
   return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE,
+            box_c == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : box_c == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+            : box_c == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1363,8 +1700,10 @@ int trtt_b200_conv3_forward(const void *x1, int c1, const void *x2, int c2, cons
   // staging: 0 cp.async, 1 TMA per tile, 2 TMA persistent (two tensor-memory
   // accumulators: 2 S n columns must fit in 512); automatic: the persistent
   // kernel where it applies, else TMA per tile, else cp.async (forward pass
-  // of the 128^3 U-Net: 1.03 / 1.37 / 1.73 ms)
-  int tma = g_conv_tma < 0 ? (encode_tiled() ? 2 : 0) : g_conv_tma;
+  // of the 128^3 U-Net: 1.03 / 1.37 / 1.73 ms); before all the z-streaming
+  // kernel where fwd_plan_z takes it
+  const bool autom = g_conv_tma < 0;
+  int tma = autom ? (encode_tiled() ? 2 : 0) : g_conv_tma;
   if (tma == 2 && pow2_cols(2 * S * n) > 512) tma = 1;
   if (a.g.rows < 256) tma = 0;  // tensors shorter than one 256-row box: cp.async
   // persistent kernel: tiles of 4 x 128 rows where two CTAs still fit on an
@@ -1373,8 +1712,11 @@ int trtt_b200_conv3_forward(const void *x1, int c1, const void *x2, int c2, cons
   // instead of 2 slab rows per output row at 128^3) and fetch each stage's
   // weights for twice the rows (forward pass 1.18 -> 1.03 ms)
   int sp = S;
+  FwdPlan zp;
+  ZArgs z;
+  if (tma == 2 && autom && fwd_plan_z(n, c1, c2, a.g, zp, z)) tma = 3;
   if (tma) {
-    const FwdPlan pl = tma == 2 ? fwd_plan_pers(n, a.groups, a.g, &sp) : fwd_plan_tma(n, a.groups, a.g);
+    const FwdPlan pl = tma == 3 ? zp : tma == 2 ? fwd_plan_pers(n, a.groups, a.g, &sp) : fwd_plan_tma(n, a.groups, a.g);
     const bool s4 = sp == 4;
     a.rh = pl.rh;
     a.cs = pl.cs;
@@ -1390,11 +1732,17 @@ int trtt_b200_conv3_forward(const void *x1, int c1, const void *x2, int c2, cons
     std::memset(&maps, 0, sizeof(maps));
     maps.tail = pl.rh % 256;
     const int tail = maps.tail ? maps.tail : 256;
-    bool ok = act_map(&maps.x1_full, x1, c1, a.g.rows, 256) && act_map(&maps.x1_tail, x1, c1, a.g.rows, tail);
-    if (c2) ok = ok && act_map(&maps.x2_full, x2, c2, a.g.rows, 256) && act_map(&maps.x2_tail, x2, c2, a.g.rows, tail);
+    const int i1 = tma == 3 ? z_channels(c1) : 8, i2 = tma == 3 ? z_channels(c2) : 8;
+    bool ok = act_map(&maps.x1_full, x1, c1, a.g.rows, 256, i1) && act_map(&maps.x1_tail, x1, c1, a.g.rows, tail, i1);
+    if (c2)
+      ok = ok && act_map(&maps.x2_full, x2, c2, a.g.rows, 256, i2) && act_map(&maps.x2_tail, x2, c2, a.g.rows, tail, i2);
     if (!ok) return fail("conv3_forward: tensor map encoding failed");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (tma == 2) {
+    if (tma == 3) {
+      auto kern = n == 16 ? k_conv3_fwd_z<3, 1, 3> : k_conv3_fwd_z<1, 2, 5>;
+      TRTT_CK(set_smem(kern, pl.smem));
+      kern<<<(unsigned)pl.tiles, z_threads(z.S, z.hw), pl.smem, st>>>(a, z, maps);
+    } else if (tma == 2) {
       auto kern = s4 ? k_conv3_fwd_pers<4> : k_conv3_fwd_pers<S>;
       TRTT_CK(set_smem(kern, pl.smem));
       // all of the SM's unified memory as shared memory, so that the
