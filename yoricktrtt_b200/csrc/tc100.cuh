@@ -48,6 +48,13 @@ __device__ __forceinline__ uint64_t sdesc_swz(uint32_t saddr, uint32_t row)
   return d;
 }
 
+// MN-major: rows (the K index) of `row` bytes as above, 8 rows per stride byte
+// offset; blocks of row / 2 elements along M or N at `lbo` bytes.
+__device__ __forceinline__ uint64_t sdesc_swz_mn(uint32_t saddr, uint32_t row, uint32_t lbo)
+{
+  return (sdesc_swz(saddr, row) & ~((uint64_t)0x3FFFu << 16)) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16);
+}
+
 // Instruction descriptor, kind::f16 with BF16 A and B and FP32 D:
 //   bits 4-5 D format (1 = F32), 7-9 A format (1 = BF16), 10-12 B format,
 //   bit 15 A major (0 = K, 1 = MN), bit 16 B major, 17-22 N >> 3, 24-28 M >> 4.

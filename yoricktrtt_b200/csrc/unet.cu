@@ -23,6 +23,8 @@
 //   the 9 (dy, dx) weight tiles of that dz; per stage 9*S MMAs of
 //   128 x N x 16.  The input gradient is the same kernel run on the output
 //   gradient with the weights transposed and flipped (tap -> 26 - tap).
+// The default kernels stream input planes along z (k_conv3_fwd_z) and fuse the
+// taps of a row and a plane (k_conv3_wgrad_rows) where they apply.
 // Weight-gradient GEMM (k_conv3_wgrad), per CTA one (dz, dy) pair and a
 // range of rows:
 //   dW[co][tap][ci] = sum_row dY[row][co] X[row + off(tap)][ci]
@@ -1168,48 +1170,236 @@ __global__ void __launch_bounds__(128) k_conv3_wgrad_tma(const WgradArgs a, cons
   }
 }
 
-__global__ void k_sum_parts(const float *__restrict__ part, int chunks, long n, float *__restrict__ out)
+// Weight gradient with the taps of a row and a plane fused into one MMA.  A CTA
+// takes one dz and a range of rows; per stage of KT rows it loads the dY rows
+// (one more on either side) and, per block of 16 to 64 input channels, the X rows
+// of that plane (wp more on either side), by TMA in the swizzle of the row width.
+// MN-major descriptors let blocks along M and N lie at any distance, so
+//   M = 128: the cout channels of dY, from the row itself and the next ones (block
+//     distance one row): the dx taps, X[r + 1 - s] for shift s;
+//   N = 3 ic: the channels of X from rows r - wp, r and r + wp: the dy taps,
+// and one MMA of 128 x 3 ic x 16 replaces nine of 64 x ic x 16 (64 output channels
+// need two, two shifts each); the rows are staged 3 times, not 9, and in 32 to
+// 128-byte instead of 16-byte pieces, which write 16 bytes of shared memory per
+// cycle (bound of k_conv3_wgrad_tma).  Thread roles, waits and the way out after a
+// failed one: k_conv3_wgrad_tma, with a whole warp issuing.
+//
+// Measured: 32 -> 32 channels at 2 x 64^3 180 -> 42 us (the MMAs' operands from
+// shared memory take 23 us, the staged rows about as long beside them).
+struct WgradRowArgs {
+  int cout, c1, c2, cin, sets;
+  float *part;          // [chunks][cout][27][cin]
+  Grid3 g;
+  long r0;              // first row summed over
+  long blocks;          // KT-row stages in all
+  int kt, steps;        // rows per stage, stages per CTA
+  int a_bytes, stage_bytes, nstg;
+  uint32_t tmem_cols;
+};
+struct WgradRowMaps {
+  CUtensorMap dy, dy_tail, x1, x1_tail, x2, x2_tail;  // 128 rows; the rest
+  int tail;                                           // rows of the X rest
+};
+
+__global__ void __launch_bounds__(128) k_conv3_wgrad_rows(const WgradRowArgs a, const __grid_constant__ WgradRowMaps maps)
 {
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int c = 0; c < chunks; ++c) s += part[(long)c * n + i];
-    out[i] = s;
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[4], empty[4], finb;
+  __shared__ uint32_t s_taddr;
+  __shared__ volatile int s_bad;
+  __shared__ int s_issued, s_consumed;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int dz = blockIdx.x, KT = a.kt, nstg = a.nstg, wp = a.g.wp;
+  const long b0 = (long)blockIdx.y * a.steps;
+  const int T = (int)max(0L, min((long)a.steps, a.blocks - b0));
+  const uint32_t sbase = tc::smem_addr(smem);
+  if (tid == 0) {
+    for (int i = 0; i < nstg; ++i) {
+      tc::mbar_init(&full[i], 1);
+      tc::mbar_init(&empty[i], 1);
+    }
+    tc::mbar_init(&finb, 1);
+    s_bad = 0;
+    s_issued = 0;
+    s_consumed = 0;
+    tc::mbar_fence_init();
+  }
+  if (warp == 0) tc::tmem_alloc(&s_taddr, a.tmem_cols);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = s_taddr;
+  const uint32_t ra = 2u * a.cout;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // producer
+      RingPos p;
+      int it = 0;
+      const uint32_t tx = (uint32_t)(KT + 8) * ra + (uint32_t)(KT + 2 * wp) * 2u * a.cin;
+      for (; it < T; ++it) {
+        if (it >= nstg && !tc::mbar_wait(&empty[p.slot], p.par ^ 1u, kWaitNs)) s_bad = 1;
+        if (s_bad) break;
+        const int q0 = (int)(a.r0 + (b0 + it) * KT), xr = q0 + (dz - 1) * (int)a.g.plane - wp;
+        uint32_t dst = sbase + (uint32_t)(p.slot * a.stage_bytes);
+        tc::mbar_arrive_expect_tx(&full[p.slot], tx);
+        for (int r = 0; r < KT; r += 128) tc::tma_load_2d(dst + (uint32_t)r * ra, &maps.dy, 0, q0 - 1 + r, &full[p.slot]);
+        tc::tma_load_2d(dst + (uint32_t)KT * ra, &maps.dy_tail, 0, q0 - 1 + KT, &full[p.slot]);
+        dst += (uint32_t)a.a_bytes;
+        for (int ch = 0; ch < a.cin;) {
+          const bool first = ch < a.c1;
+          const int ic = z_channels(first ? a.c1 : a.c2), x = first ? ch : ch - a.c1, rows = KT + 2 * wp;
+          const uint32_t rb = 2u * ic;
+          for (int r = 0; r < rows; r += 128)
+            tc::tma_load_2d(dst + (uint32_t)r * rb,
+                            first ? (rows - r >= 128 ? &maps.x1 : &maps.x1_tail) : (rows - r >= 128 ? &maps.x2 : &maps.x2_tail),
+                            x, xr + r, &full[p.slot]);
+          dst += ((uint32_t)rows * rb + 1023u) & ~1023u;
+          ch += ic;
+        }
+        p.next(nstg);
+      }
+      s_issued = it;
+    }
+  } else if (warp == 1) {
+    // MMA issuer (the whole warp, every value the same in its lanes)
+    auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
+    RingPos p;
+    int it = 0;
+    for (; it < T; ++it) {
+      const bool in = tc::mbar_wait(&full[p.slot], p.par, kWaitNs);
+      if (!__all_sync(0xffffffffu, in && !s_bad)) {
+        s_bad = 1;
+        break;
+      }
+      tc::fence_after_sync();
+      const uint32_t as = sbase + (uint32_t)(p.slot * a.stage_bytes);
+      uint32_t bs = as + (uint32_t)a.a_bytes;
+      for (int ch = 0; ch < a.cin;) {
+        const int ic = z_channels(ch < a.c1 ? a.c1 : a.c2);
+        const uint32_t rb = uniform(2u * ic), idesc = uniform(tc::idesc_bf16(128, 3 * ic, 1, 1));
+        const uint64_t bd = tc::sdesc_swz_mn(bs, rb, (uint32_t)wp * rb);
+        for (int set = 0; set < a.sets; ++set) {
+          const uint64_t ad = tc::sdesc_swz_mn(as + 2u * set * ra, ra, ra);
+          const uint32_t alo = uniform((uint32_t)ad), ahi = uniform((uint32_t)(ad >> 32));
+          const uint32_t blo = uniform((uint32_t)bd), bhi = uniform((uint32_t)(bd >> 32));
+          const uint32_t acc = uniform(tmem + (uint32_t)(3 * (set * a.cin + ch)));
+          // 16 rows per MMA; descriptors count 16 bytes
+#pragma unroll 8
+          for (int ks = 0; ks < KT / 16; ++ks)
+            tc::mma_bf16_warp(acc, alo + (uint32_t)ks * ra, ahi, blo + (uint32_t)ks * rb, bhi, idesc,
+                              (it > 0 || ks > 0) ? 1u : 0u);
+        }
+        bs += ((uint32_t)(KT + 2 * wp) * rb + 1023u) & ~1023u;
+        ch += ic;
+      }
+      tc::mma_commit_warp(&empty[p.slot]);
+      p.next(nstg);
+    }
+    if (lane == 0) s_consumed = it;
+    tc::mma_commit_warp(&finb);  // arrives once every MMA issued above has completed
+  }
+  const bool fin_ok = tc::mbar_wait(&finb, 0, kWaitNs);
+  __syncthreads();
+  const bool bad = s_bad || !fin_ok;
+  if (!bad) {
+    tc::fence_after_sync();
+    // accumulator row s cout + co: shift s of channel co
+    const int row = 32 * warp + lane;
+    for (int set = 0; set < a.sets; ++set) {
+      const int s = 2 * set + row / a.cout, co = row % a.cout;
+      if (__all_sync(0xffffffffu, s > 2)) continue;
+      float *dst = a.part + (((long)blockIdx.y * a.cout + co) * 27 + dz * 9 + 2 - s) * a.cin;
+      for (int ch = 0; ch < a.cin;) {
+        const int ic = z_channels(ch < a.c1 ? a.c1 : a.c2);
+        for (int dy = 0; dy < 3; ++dy)
+          for (int j = 0; j < ic; j += 16) {
+            float v[16];
+            tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(3 * (set * a.cin + ch) + dy * ic + j), v);
+            if (s <= 2) {
+              float4 *o = reinterpret_cast<float4 *>(dst + (long)dy * 3 * a.cin + ch + j);
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                o[i] = T > 0 ? make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+          }
+        ch += ic;
+      }
+    }
+  } else if (tid == 0) {
+    // copies issued for stages the MMAs never consumed
+    for (int it = s_consumed; it < s_issued; ++it)
+      tc::mbar_wait(&full[it % nstg], (uint32_t)(it / nstg) & 1u, kWaitNs);
+    atomicExch(&g_unet_err, 1);
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, a.tmem_cols);
   }
 }
 
-// per-channel sum over all rows (bias gradient); rows of the border are zero
-__global__ void k_chan_sum(const bf16 *__restrict__ g, long rows, int c, float *__restrict__ out)
+// out[i] = sum over chunks of part[chunk][i]; 32 outputs and 8 threads per output
+// in a block (one thread per output was a chain of ~100 loads: 11.4 -> 4.1 us for 98
+// chunks of 27648).  Clears
+// `zero` (nz floats), which the next kernel adds into.
+__global__ void __launch_bounds__(256) k_sum_parts(const float *__restrict__ part, int chunks, long n,
+                                                   float *__restrict__ out, float *zero, int nz)
 {
-  extern __shared__ float acc[];
-  for (int i = threadIdx.x; i < c; i += blockDim.x) acc[i] = 0.f;
-  __syncthreads();
-  const int nch = c / 8;
-  float part[8];
-  int cur = -1;
-  for (int i = 0; i < 8; ++i) part[i] = 0.f;
-  // consecutive threads take consecutive 16-byte chunks; each thread keeps
-  // the chunk index fixed when the stride is a multiple of nch
-  const long total = rows * nch;
-  const long stride = (long)gridDim.x * blockDim.x;
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += stride) {
-    const int ch = (int)(e % nch);
-    if (ch != cur) {
-      if (cur >= 0)
-        for (int i = 0; i < 8; ++i) atomicAdd(&acc[cur * 8 + i], part[i]), part[i] = 0.f;
-      cur = ch;
+  __shared__ float sh[8][33];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && zero && threadIdx.x < nz) zero[threadIdx.x] = 0.f;
+  for (long b = (long)blockIdx.x * 32; b < n; b += (long)gridDim.x * 32) {
+    float s = 0.f;
+    if (b + x < n)
+      for (int c = y; c < chunks; c += 8) s += part[(long)c * n + b + x];
+    sh[y][x] = s;
+    __syncthreads();
+    if (y == 0 && b + x < n) {
+      s = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s += sh[k][x];
+      out[b + x] = s;
     }
-    const uint4 q = reinterpret_cast<const uint4 *>(g)[e];
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = unpack_bf16x2(w[i]);
-      part[2 * i] += f.x;
-      part[2 * i + 1] += f.y;
+    __syncthreads();
+  }
+}
+
+// per-channel sum over all rows (bias gradient); rows of the border are zero.
+// A thread keeps its 8 channels: threads of a block are (row, chunk) pairs (a
+// 64-bit remainder per 16 bytes and shared atomics before: 20 -> 7 us for 37 MB).
+__global__ void __launch_bounds__(256) k_chan_sum(const bf16 *__restrict__ g, long rows, int c, float *__restrict__ out)
+{
+  __shared__ float acc[256][9];
+  const int nch = c / 8, ch = threadIdx.x % nch, per = 256 / nch, r0 = threadIdx.x / nch;
+  float part[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) part[i] = 0.f;
+  if (r0 < per) {
+    const uint4 *src = reinterpret_cast<const uint4 *>(g) + ch;
+    const long hop = (long)gridDim.x * per;
+#pragma unroll 4
+    for (long r = (long)blockIdx.x * per + r0; r < rows; r += hop) {
+      const uint4 q = __ldg(src + r * nch);
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = unpack_bf16x2(w[i]);
+        part[2 * i] += f.x;
+        part[2 * i + 1] += f.y;
+      }
     }
   }
-  if (cur >= 0)
-    for (int i = 0; i < 8; ++i) atomicAdd(&acc[cur * 8 + i], part[i]);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[threadIdx.x][i] = part[i];
   __syncthreads();
-  for (int i = threadIdx.x; i < c; i += blockDim.x) atomicAdd(&out[i], acc[i]);
+  // channel k: the block's partial sums of its chunk
+  for (int k = threadIdx.x; k < c; k += 256) {
+    float s = 0.f;
+    for (int r = 0; r < per; ++r) s += acc[r * nch + k / 8][k & 7];
+    atomicAdd(&out[k], s);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1661,6 +1851,51 @@ WgradPlan wgrad_plan(int cout, int cin, const Grid3 &g, bool tma = false)
   return p;
 }
 
+// Layout of k_conv3_wgrad_rows; false where it does not apply.  256 rows per stage
+// where three stages leave room for two CTAs on an SM, else 128 (the X slab's 2 wp
+// extra rows weigh more, but two CTAs overlap their waits); one wave of CTAs.  Below
+// 4096 rows the 9 per-tap CTAs of a range are faster than 3 (64 -> 64 at 8^3 25.6
+// us against 29.7; at 16^3 all are faster here).
+struct WgradRowPlan {
+  int kt, a_bytes, stage_bytes, nstg, smem, sets;
+  long chunks, steps, blocks;
+  uint32_t tmem_cols;
+};
+bool wgrad_row_plan(int cout, int c1, int c2, const Grid3 &g, WgradRowPlan &p)
+{
+  const int cin = c1 + c2;
+  if (cout != 16 && cout != 32 && cout != 64) return false;
+  p.sets = cout == 64 ? 2 : 1;
+  if (p.sets * 3 * cin > 512 || g.wp >= 2048 || g.rows < 4096 || g.rows + 4096 + g.plane >= 0x7FFFFFFFL) return false;
+  p.tmem_cols = pow2_cols(p.sets * 3 * cin);
+  auto layout = [&](int kt) {
+    auto up = [](int b) { return (b + 1023) & ~1023; };
+    p.kt = kt;
+    p.a_bytes = up((kt + 8) * 2 * cout);
+    p.stage_bytes = p.a_bytes;
+    for (int ch = 0; ch < cin;) {
+      const int ic = z_channels(ch < c1 ? c1 : c2);
+      p.stage_bytes += up((kt + 2 * g.wp) * 2 * ic);
+      ch += ic;
+    }
+  };
+  const bool pair = p.tmem_cols <= 256;
+  const int half = 110 * 1024, whole = 224 * 1024;
+  layout(256);
+  if (!(pair && 3 * p.stage_bytes <= half)) layout(128);
+  const int room = pair && 2 * p.stage_bytes <= half ? half : whole;
+  p.nstg = std::min(4, room / p.stage_bytes);
+  if (p.nstg < 2) return false;
+  p.smem = residency_smem(p.nstg * p.stage_bytes, p.tmem_cols);
+  if (p.smem > 226 * 1024) return false;
+  p.blocks = (g.rows - 2 * g.plane + p.kt - 1) / p.kt;
+  const long ctas = 148L * (2 * (p.smem + 2048) <= 227 * 1024 && pair ? 2 : 1);
+  const long most = std::min(p.blocks, std::max(1L, ctas / 3));
+  p.steps = (p.blocks + most - 1) / most;
+  p.chunks = (p.blocks + p.steps - 1) / p.steps;
+  return true;
+}
+
 template <typename K>
 cudaError_t set_smem(K kern, int bytes)
 {
@@ -1830,9 +2065,11 @@ int trtt_b200_conv3_plan_info(int which, int cin, int cout, int nb, int d, int h
 size_t trtt_b200_conv3_wgrad_scratch(int cout, int cin, int nb, int d, int h, int w)
 {
   if (!grid_ok(nb, d, h, w) || cout <= 0 || cin <= 0 || cout % 8 || cin % 8) return 0;
-  // enough for either staging
+  // enough for every kernel
   const Grid3 g = make_grid(nb, d, h, w);
-  const long chunks = std::max(wgrad_plan(cout, cin, g, false).chunks, wgrad_plan(cout, cin, g, true).chunks);
+  long chunks = std::max(wgrad_plan(cout, cin, g, false).chunks, wgrad_plan(cout, cin, g, true).chunks);
+  // (k_conv3_wgrad_rows: at most two CTAs per SM over three dz)
+  chunks = std::max(chunks, std::min((g.rows - 2 * g.plane + 127) / 128, 2L * 148 / 3));
   return (size_t)chunks * cout * 27 * cin * sizeof(float);
 }
 
@@ -1862,43 +2099,72 @@ int trtt_b200_conv3_wgrad(const void *dy, int cout, const void *x1, int c1, cons
   const bool tma = g_conv_tma != 0 && encode_tiled() && a.g.rows >= 256 && a.g.rows + 512 < 0x7FFFFFFFL &&
                    !(reinterpret_cast<uintptr_t>(dy) & 15) && !(reinterpret_cast<uintptr_t>(x1) & 15) &&
                    !(c2 && (reinterpret_cast<uintptr_t>(x2) & 15));
-  const WgradPlan pl = wgrad_plan(cout, cin, a.g, tma);
-  if (pl.steps > 0x7FFFFFFFL) return fail("conv3_wgrad: too many rows");
-  const long chunks = pl.chunks;
-  a.kt = pl.kt;
-  a.steps = (int)pl.steps;
-  const size_t need = (size_t)chunks * cout * 27 * cin * sizeof(float);
-  if (scratch_bytes < need) return fail("conv3_wgrad: scratch too small");
-  a.part = static_cast<float *>(scratch);
-  a.csa = pl.csa;
-  a.csb = pl.csb;
-  a.a_bytes = pl.a_bytes;
-  a.b_bytes = pl.b_bytes;
-  a.nstg = pl.nstg;
-  a.tmem_cols = pl.tmem_cols;
-  const int smem = pl.smem;
-  if (smem > 227 * 1024) return fail("conv3_wgrad: stage too large");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  dim3 grid(9, (unsigned)chunks);
-  if (tma) {
-    WgradMaps maps;
+  a.part = static_cast<float *>(scratch);
+  WgradRowPlan rp;
+  long chunks = 0;
+  if (tma && g_conv_tma < 0 && wgrad_row_plan(cout, c1, c2, a.g, rp) &&
+      scratch_bytes >= (size_t)rp.chunks * cout * 27 * cin * sizeof(float)) {
+    chunks = rp.chunks;
+    WgradRowArgs r;
+    r.cout = cout; r.c1 = c1; r.c2 = c2; r.cin = cin; r.sets = rp.sets;
+    r.part = a.part;
+    r.g = a.g;
+    r.r0 = a.r0;
+    r.blocks = rp.blocks;
+    r.kt = rp.kt;
+    r.steps = (int)rp.steps;
+    r.a_bytes = rp.a_bytes;
+    r.stage_bytes = rp.stage_bytes;
+    r.nstg = rp.nstg;
+    r.tmem_cols = rp.tmem_cols;
+    WgradRowMaps maps;
     std::memset(&maps, 0, sizeof(maps));
-    bool ok = act_map(&maps.dy, dy, cout, a.g.rows, 128) && act_map(&maps.x1, x1, c1, a.g.rows, 128) &&
-              act_map(&maps.x1_tail, x1, c1, a.g.rows, 2);
-    if (c2) ok = ok && act_map(&maps.x2, x2, c2, a.g.rows, 128) && act_map(&maps.x2_tail, x2, c2, a.g.rows, 2);
+    maps.tail = (2 * a.g.wp) % 128;
+    const int tail = maps.tail ? maps.tail : 128, i1 = z_channels(c1), i2 = c2 ? z_channels(c2) : 16;
+    bool ok = act_map(&maps.dy, dy, cout, a.g.rows, 128, cout) && act_map(&maps.dy_tail, dy, cout, a.g.rows, 8, cout) &&
+              act_map(&maps.x1, x1, c1, a.g.rows, 128, i1) && act_map(&maps.x1_tail, x1, c1, a.g.rows, tail, i1);
+    if (c2) ok = ok && act_map(&maps.x2, x2, c2, a.g.rows, 128, i2) && act_map(&maps.x2_tail, x2, c2, a.g.rows, tail, i2);
     if (!ok) return fail("conv3_wgrad: tensor map encoding failed");
-    TRTT_CK(set_smem(k_conv3_wgrad_tma, smem));
-    k_conv3_wgrad_tma<<<grid, 128, smem, st>>>(a, maps);
+    TRTT_CK(set_smem(k_conv3_wgrad_rows, rp.smem));
+    TRTT_CK(cudaFuncSetAttribute(k_conv3_wgrad_rows, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    k_conv3_wgrad_rows<<<dim3(3, (unsigned)chunks), 128, rp.smem, st>>>(r, maps);
   } else {
-    TRTT_CK(set_smem(k_conv3_wgrad, smem));
-    k_conv3_wgrad<<<grid, 128, smem, st>>>(a);
+    const WgradPlan pl = wgrad_plan(cout, cin, a.g, tma);
+    if (pl.steps > 0x7FFFFFFFL) return fail("conv3_wgrad: too many rows");
+    chunks = pl.chunks;
+    a.kt = pl.kt;
+    a.steps = (int)pl.steps;
+    const size_t need = (size_t)chunks * cout * 27 * cin * sizeof(float);
+    if (scratch_bytes < need) return fail("conv3_wgrad: scratch too small");
+    a.csa = pl.csa;
+    a.csb = pl.csb;
+    a.a_bytes = pl.a_bytes;
+    a.b_bytes = pl.b_bytes;
+    a.nstg = pl.nstg;
+    a.tmem_cols = pl.tmem_cols;
+    const int smem = pl.smem;
+    if (smem > 227 * 1024) return fail("conv3_wgrad: stage too large");
+    dim3 grid(9, (unsigned)chunks);
+    if (tma) {
+      WgradMaps maps;
+      std::memset(&maps, 0, sizeof(maps));
+      bool ok = act_map(&maps.dy, dy, cout, a.g.rows, 128) && act_map(&maps.x1, x1, c1, a.g.rows, 128) &&
+                act_map(&maps.x1_tail, x1, c1, a.g.rows, 2);
+      if (c2) ok = ok && act_map(&maps.x2, x2, c2, a.g.rows, 128) && act_map(&maps.x2_tail, x2, c2, a.g.rows, 2);
+      if (!ok) return fail("conv3_wgrad: tensor map encoding failed");
+      TRTT_CK(set_smem(k_conv3_wgrad_tma, smem));
+      k_conv3_wgrad_tma<<<grid, 128, smem, st>>>(a, maps);
+    } else {
+      TRTT_CK(set_smem(k_conv3_wgrad, smem));
+      k_conv3_wgrad<<<grid, 128, smem, st>>>(a);
+    }
   }
   const long nw = (long)cout * 27 * cin;
-  k_sum_parts<<<grid_for(nw), 256, 0, st>>>(a.part, (int)chunks, nw, dw);
+  k_sum_parts<<<(unsigned)std::min((nw + 31) / 32, 148L * 8), 256, 0, st>>>(a.part, (int)chunks, nw, dw, db, cout);
   count_launch(2);
   if (db) {
-    TRTT_CK(cudaMemsetAsync(db, 0, sizeof(float) * cout, st));
-    k_chan_sum<<<148 * 4, 256, sizeof(float) * cout, st>>>(a.dy, a.g.rows, cout, db);
+    k_chan_sum<<<148 * 4, 256, 0, st>>>(a.dy, a.g.rows, cout, db);
     count_launch();
   }
   TRTT_CK(cudaGetLastError());
