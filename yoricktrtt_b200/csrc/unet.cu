@@ -622,7 +622,11 @@ struct ZArgs {
 
 constexpr int kZStages = 12;
 
-__host__ __device__ constexpr int z_threads(int S, int HW) { return 128 * S * HW + 32 + 32 * S; }
+constexpr int kZIssue = 3;  // MMA warps
+// sets of epilogue warps, taking output planes in turn: an epilogue is a chain of
+// about 1500 cycles, longer than a plane of 128 rows takes the tensor core
+__host__ __device__ constexpr int z_sets(int S) { return S == 1 ? 2 : 1; }
+__host__ __device__ constexpr int z_threads(int S, int HW) { return 128 * S * HW * z_sets(S) + 32 + 32 * kZIssue; }
 // Channels per row of a stage: 32, 64 or 128 bytes, the swizzle's widths.
 __host__ __device__ inline int z_channels(int c) { return c % 64 == 0 ? 64 : c % 32 == 0 ? 32 : 16; }
 
@@ -643,16 +647,16 @@ struct RingPos {
 template <int S, int HW, int NB>
 __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdArgs a, const ZArgs z, const __grid_constant__ FwdMaps maps)
 {
+  constexpr int ES = z_sets(S), EP = 4 * S * HW, EW = EP * ES;  // epilogue warps (EP a set); then the producer and the issuers
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t full[kZStages], empty[kZStages], accf[NB], acce[NB], edgeb, finb;
+  __shared__ __align__(8) uint64_t full[kZStages], empty[kZStages], accf[NB], acce[NB], edgeb[ES], finb;
   __shared__ uint32_t s_taddr;
   __shared__ volatile int s_bad;
   __shared__ int s_issued, s_consumed;
-  constexpr int EW = 4 * S * HW;  // epilogue warps; then the producer and S issuers
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int G = a.groups, n = a.n, nstg = a.nstg, wp = a.g.wp;
   const uint32_t sbase = tc::smem_addr(smem), ring = sbase + (uint32_t)(z.w_bytes + z.edge_bytes);
-  float *edge = reinterpret_cast<float *>(smem + z.w_bytes);  // [2][4 S + 2][2][n]
+  float *edge = reinterpret_cast<float *>(smem + z.w_bytes);  // [set][2][4 S + 2][2][n]
   const int unit = blockIdx.x, seg = unit % z.segs, tile = (unit / z.segs) % z.tiles, vol = unit / (z.segs * z.tiles);
   const int za = 1 + seg * z.len, zb = min(za + z.len, a.g.d + 1);
   const int zlo = max(za - 1, 1), zhi = min(zb, a.g.d);  // input planes
@@ -662,14 +666,14 @@ __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdAr
   if (tid == 0) {
     for (int i = 0; i < nstg; ++i) {
       tc::mbar_init(&full[i], 1);
-      tc::mbar_init(&empty[i], S);
+      tc::mbar_init(&empty[i], kZIssue);
     }
     for (int b = 0; b < NB; ++b) {
       tc::mbar_init(&accf[b], S);
-      tc::mbar_init(&acce[b], EW);
+      tc::mbar_init(&acce[b], EP);
     }
-    tc::mbar_init(&edgeb, EW);
-    tc::mbar_init(&finb, S);
+    for (int e = 0; e < ES; ++e) tc::mbar_init(&edgeb[e], EP);
+    tc::mbar_init(&finb, kZIssue);
     s_bad = 0;
     s_issued = 0;
     s_consumed = 0;
@@ -716,9 +720,10 @@ __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdAr
       s_issued = c;
     }
   } else if (warp >= EW + 1) {
-    // MMA issuer of sub-tile s (the whole warp, every value the same in its lanes)
+    // MMA issuer (the whole warp, every value the same in its lanes)
     const uint32_t idesc = tc::idesc_bf16(128, 3 * n, 0, 0);
-    const int s = warp - (EW + 1);
+    // S = 3: of sub-tile s; S = 1: of the output planes zo = own mod 3
+    const int s = S == 3 ? warp - (EW + 1) : 0, own = warp - (EW + 1);
     auto uniform = [](uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); };
     const uint32_t bstep = uniform((uint32_t)(6 * G) * cols);
     RingPos p;
@@ -727,7 +732,13 @@ __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdAr
     // accumulators of zi - 1, zi, zi + 1
     int b2 = (zlo + NB - 1) % NB, b1 = zlo % NB, b0 = (zlo + 1) % NB;
     for (int zi = zlo; zi <= zhi && ok; ++zi) {
-      const bool v2 = zi - 1 >= za, v1 = zi >= za && zi < zb, v0 = zi + 1 < zb;
+      bool v2 = zi - 1 >= za, v1 = zi >= za && zi < zb, v0 = zi + 1 < zb;
+      if (S == 1) {
+        const int m = zi % 3;
+        v2 = v2 && m == (own + 1) % 3;
+        v1 = v1 && m == own;
+        v0 = v0 && m == (own + 2) % 3;
+      }
       // output zi + 1 starts here; output 1 already with plane 1 (0 is left out)
       const uint32_t acc[3] = {uniform(tmem + (uint32_t)(b0 * S + s) * cols), uniform(tmem + (uint32_t)(b1 * S + s) * cols),
                                uniform(tmem + (uint32_t)(b2 * S + s) * cols)};
@@ -785,16 +796,16 @@ __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdAr
       b0 = b0 + 1 == NB ? 0 : b0 + 1;
     }
     if (!ok) s_bad = 1;
-    if (s == 0 && lane == 0) s_consumed = used;
+    if (own == 0 && lane == 0) s_consumed = used;
     tc::mma_commit_warp(&finb);  // arrives once every MMA issued above has completed
   } else {
     // epilogue
-    const int q = warp & 3, s = (warp >> 2) % S, j = 16 * ((warp >> 2) / S);
+    const int set = warp / EP, we = warp % EP, q = we & 3, s = (we >> 2) % S, j = 16 * ((we >> 2) / S);
     const int blk = 4 * s + q;  // blocks of 32 rows in order
     const int ip = m0 + 32 * blk + lane, y = ip / wp, x = ip - y * wp, r = 32 * blk + lane;
     const bool inside = r > 0 && r < 128 * S - 1 && y >= 1 && y <= a.g.h && x >= 1 && x <= a.g.w;
-    for (int zo = za; zo < zb; ++zo) {
-      const int u = zo - za;
+    for (int zo = za + set; zo < zb; zo += ES) {
+      const int u = zo - za, turn = u / ES;
       const bool full_ok = tc::mbar_wait(&accf[zo % NB], (uint32_t)(u / NB) & 1u, kWaitNs);
       if (!__all_sync(0xffffffffu, full_ok)) {
         s_bad = 1;
@@ -802,7 +813,7 @@ __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdAr
       }
       tc::fence_after_sync();
       const uint32_t acc = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)((zo % NB) * S + s) * cols;
-      float *ed = edge + (u & 1) * (4 * S + 2) * 2 * n;
+      float *ed = edge + (2 * set + (turn & 1)) * (4 * S + 2) * 2 * n;
       float v[3][16];
       tc::tmem_ld16x3(acc + (uint32_t)j, acc + (uint32_t)(n + j), acc + (uint32_t)(2 * n + j), v);
       tc::fence_before_sync();
@@ -820,13 +831,13 @@ __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdAr
         for (int i = 0; i < 4; ++i) o[i] = make_float4(v[2][4 * i], v[2][4 * i + 1], v[2][4 * i + 2], v[2][4 * i + 3]);
       }
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&edgeb);
+      if (lane == 0) tc::mbar_arrive(&edgeb[set]);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         v[0][i] = __shfl_up_sync(0xffffffffu, v[0][i], 1);
         v[2][i] = __shfl_down_sync(0xffffffffu, v[2][i], 1);
       }
-      const bool edge_ok = tc::mbar_wait(&edgeb, (uint32_t)u & 1u, kWaitNs);
+      const bool edge_ok = tc::mbar_wait(&edgeb[set], (uint32_t)turn & 1u, kWaitNs);
       if (!__all_sync(0xffffffffu, edge_ok)) {
         s_bad = 1;
         break;
@@ -1735,7 +1746,7 @@ bool fwd_plan_z(int n, int c1, int c2, const Grid3 &g, FwdPlan &p, ZArgs &z)
   p.cs = 0;
   p.stage_bytes = ((p.rh * 2 * ic + 1023) / 1024) * 1024;
   z.w_bytes = ((27 * groups * 16 * n * 2 + 1023) / 1024) * 1024;
-  z.edge_bytes = ((2 * (4 * z.S + 2) * 2 * n * 4 + 1023) / 1024) * 1024;
+  z.edge_bytes = ((z_sets(z.S) * 2 * (4 * z.S + 2) * 2 * n * 4 + 1023) / 1024) * 1024;
   const int room = 224 * 1024 - z.w_bytes - z.edge_bytes;
   p.nstg = std::min(kZStages, room / p.stage_bytes);
   if (room <= 0 || p.nstg < 2) return false;
