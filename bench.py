@@ -222,12 +222,12 @@ def run_reference(args):
 # B200 arm
 # ---------------------------------------------------------------------------
 # names of the kernels the step launches (per direction), for the roofline:
-# the group kernels when the scan's views group by turns of the grid, else
-# the per-view kernels
-KERNELS = {True: ("k_fwd3d_group (direct, view groups x detector-row bands)",
+# over groups of views when the scan's views group by turns of the grid, else
+# view by view
+KERNELS = {True: ("k_fwd3d_sweep (direct, line sweeps, view groups x detector tiles)",
                   "k_back3d_group (transpose, column orbits)"),
-           False: ("k_fwd3d_band_fast (direct, detector-row bands)",
-                   "k_back3d_col_fast (transpose, column gather)")}
+           False: ("k_fwd3d_sweep (direct, line sweeps, views x detector tiles)",
+                   "k_back3d_gather (transpose, four columns per warp)")}
 PARITY_VIEWS = (0, 137, 271)
 
 
@@ -416,7 +416,7 @@ def run_b200(args):
         pms = max_over_ranks(pms)
         per_view = {"value": 2 * VIEWS * world * psteps / (pms / 1e3), "unit": "projections/s",
                     "fwd_ms": statistics.mean(pfwd), "back_ms": statistics.mean(pback),
-                    "steps": psteps, "kernels": "k_fwd3d_band_fast + k_back3d_col_fast"}
+                    "steps": psteps, "kernels": "k_fwd3d_sweep + k_back3d_gather"}
         pr.set_symmetry(True)  # back to the default group kernels
 
     # the same pair on a dense volume (every voxel non-zero, as a
@@ -449,7 +449,7 @@ def run_b200(args):
         table_model = {"value": 2 * VIEWS * world * tsteps / (tms / 1e3), "unit": "projections/s",
                        "fwd_ms": statistics.mean(tfwd), "back_ms": statistics.mean(tback),
                        "steps": tsteps, "footprint": "table of 10001 samples (FP64), per-view kernels",
-                       "kernels": "k_fwd3d_band_table + k_back3d_col_fast (table model)"}
+                       "kernels": "k_fwd3d_sweep + k_back3d_gather (table model)"}
         prt.close()
 
     # roofline of the dominant kernel: algorithmic bytes per launch (per-view

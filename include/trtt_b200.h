@@ -231,7 +231,7 @@ int trtt_b200_plan3d_set_tiles(trtt_b200_plan3d *plan, int band_rows, int warps)
  * pair kernel's shared memory (band + 2 profiles per warp) does not fit. */
 int trtt_b200_plan3d_set_columns(trtt_b200_plan3d *plan, int cols);
 
-/* Weighted least-squares data term in one persistent launch.  No single
+/* Weighted least-squares data term in one call.  No single
  * counterpart in the reference: it is the cost evaluation of its 4D
  * reconstruction (Tomography_4D/Ytrtt4D_optim.i:87-223) with the per-gate
  * projection of Ytrtt_3D_projectors.i:254-375.  For the plan's views (gates
@@ -241,8 +241,10 @@ int trtt_b200_plan3d_set_columns(trtt_b200_plan3d *plan, int cols);
  * vol and grad: device, column layout (TRTT_B200_LAYOUT_COLUMNS), gates
  * stacked; y and w: device [view][nv][nu] (w NULL: unit weights); cost:
  * device, one double.  Closed-form model, column-factorised views (else
- * -1).  One cooperative launch of resident CTAs draws (view, band) items,
- * then (gate, column block) items from a device queue; a column item waits,
+ * -1).  Three launches (direct projection, residual with its cost,
+ * transpose); with a shape set by plan3d_set_persistent one cooperative launch
+ * of resident CTAs that draws (view, band) items, then (gate, column block)
+ * items from a device queue; a column item waits,
  * bounded by the plan's wait limit, for every band item; a wait that runs
  * out makes the next plan3d_status call fail ("bounded device wait ran
  * out") and the launch returns early.

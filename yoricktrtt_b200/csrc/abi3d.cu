@@ -400,7 +400,7 @@ extern "C" int trtt_b200_plan3d_wls_grad(trtt_b200_plan3d *pl, const float *vol,
   const Params3D &P = pl->P;
   if (!pl->wls_set && pl->wls_extra == 0 && pl->band_rows > 0 && pl->nviews <= 65535) {
     // direct projection, residual with its cost, transpose: three launches, each
-    // at its own shape.  10 gates of 128 x 128 x 64, 347 views on 256^2: 24.4 ms;
+    // at its own shape.  10 gates of 128 x 128 x 64, 347 views on 256^2: 20.5 ms;
     // the persistent launch 26.0 at its best shape and 28.5-33 at its default
     // one.  The direct projection is the band kernel, whose FP32 sums are the
     // persistent launch's: the FP64 cost shows their rounding (8e-8 below the

@@ -594,7 +594,8 @@ __global__ void __launch_bounds__(192) k_conv3_fwd_pers(const FwdArgs a, const _
 // rows, out[r] = D_0[r-1] + D_1[r] + D_2[r+1] (rows are tensor-memory lanes:
 // shuffles, and the rows at a warp's edge through shared memory): 9 MMAs per 16
 // channels and 128 rows, not 27.  All weights stay in shared memory.
-//   4 S HW warps: epilogue, warp (s, q, j): 32 rows 128 s + 32 q, channels
+//   4 S HW warps (S = 1: two such sets, by turns): epilogue, warp (s, q, j): 32
+//     rows 128 s + 32 q, channels
 //     [j, j + 16): it takes its three blocks to registers, which frees the
 //     buffer, and then exchanges rows and writes;
 //   warp EW, one thread: producer, stages (input plane, 16 to 64 channels) into
@@ -602,18 +603,19 @@ __global__ void __launch_bounds__(192) k_conv3_fwd_pers(const FwdArgs a, const _
 //     that width.  Boxes of 8 channels would write 16 bytes of shared memory per
 //     cycle and fetch each 32-byte sector twice (120 us of the first layer below
 //     by themselves);
-//   S warps: MMA issuers of one sub-tile each (an MMA takes a warp about 60
-//     cycles to issue, the tensor core about 45).  Per stage dz = 2, 1, 0; the
+//   three warps: MMA issuers, of one sub-tile each (S = 3) or of every third
+//     output plane (S = 1): an MMA takes a warp about 60 cycles to issue, the
+//     tensor core about 45.  Per stage dz = 2, 1, 0; the
 //     plane's last stage completes output z - 1 (`accf`), the first dz = 0 of a
 //     plane waits for the epilogue that had the buffer before (`acce`).
 // Input planes 0 and d + 1 are zero and left out.  Waits and the way out after a
 // failed one: as k_conv3_fwd_pers (the epilogue warps meet on bounded mbarriers,
 // never on a block barrier).
 //
-// Measured against k_conv3_fwd_pers: 48 -> 16 channels at 128^3 269 -> 127 us, 32
-// -> 32 at 2 x 64^3 66 -> 54 us.  Bounds: the first 100 us of MMAs (A from shared
-// memory: 4 KB each for 3n columns), staging 54 us beside them; the second the
-// chain of waits per plane (23 us without any load or MMA) and 41 us of MMAs.
+// Measured against k_conv3_fwd_pers: 48 -> 16 channels at 128^3 269 -> 128 us, 32
+// -> 32 at 2 x 64^3 66 -> 43 us.  Bounds: the first about 100 us of MMAs (A from
+// shared memory: 4 KB each for 3n columns), staging 54 us beside them; the second
+// the chain of waits per plane (23 us without any load or MMA).
 struct ZArgs {
   int S, tiles, segs, len;    // sub-tiles; tiles per plane, z segments per volume and their length
   int hw;                     // epilogue warps per 32 rows, n / 16
@@ -764,8 +766,9 @@ __global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdAr
                               bhi, idesc, add);
           };
           const bool wait = g == 0 && v0 && zi + 1 - NB >= za;
-          // MMAs of the three output planes alternate: those into one accumulator
-          // follow each other by their latency
+          // (one MMA of 9n columns for the three output planes measured 122 -> 116 us on
+          // 48 -> 16 at 128^3 and 10% slower at 64^3 and below: its weights in every
+          // rotation take longer to load and leave the ring a stage less)
 #pragma unroll
           for (int dy = 0; dy < 3; ++dy) {
             if (v2) mma(2, dy, 1u);

@@ -125,7 +125,7 @@ class Projector3D:
             "trtt_b200_plan3d_set_group_tiles")
 
     def wls_grad(self, vol, y, grad, w=None, cost=None):
-        """One persistent launch: grad += H^T W (H vol - y), returns the
+        """The data term in one call: grad += H^T W (H vol - y), returns the
         device FP64 cost 1/2 sum W (H vol - y)^2 (columns layout, gates
         stacked; y, w: (nviews, nv, nu) float32)."""
         torch = _torch()
