@@ -36,7 +36,7 @@ __device__ __forceinline__ int foot2d(const Params2D &P, const View2D &V, int i,
     double delta_v = dsqrt(dadd(1.0, ddiv(dmul(vca8, vca8), V.a4sqr)));
     f.rho0 = dmul(dmul(P.rho0_init, magn), delta_v);
     h = dmul(dmul(P.h_init, magn), delta_v);
-    scl = P.table ? ddiv(1.0, dmul(h, P.step)) : ddiv(1.0, h);
+    scl = __drcp_rn(P.table ? dmul(h, P.step) : h);
     hs = dmul(P.hs0, h);
   } else {
     // plugin/trtt_2D_projectors.c:222-226
