@@ -259,6 +259,14 @@ int trtt_b200_plan3d_wls_grad(trtt_b200_plan3d *plan, const float *vol, const fl
 int trtt_b200_plan3d_set_persistent(trtt_b200_plan3d *plan, int band_rows, int ctas_per_sm,
                                     double wait_seconds, int extra_wait);
 
+/* Host-only: what the closed-form sweep and gather kernels take as bounds of
+ * these views, info[5] = {detector rows of one voxel column (0: these views
+ * keep the general kernels), first and last + 1 cell and row that a footprint
+ * can reach}. */
+int trtt_b200_sweep_bounds_info(int geometry, long nx, long ny, long nz, double s_scl, int s_deg, long nu,
+                                long nv, double u_scl, double v_scl, long nviews, const double *xos,
+                                const double *xsd, long *info);
+
 /* 1 if every view of the plan uses the column-factorised kernels. */
 int trtt_b200_plan3d_factorized(const trtt_b200_plan3d *plan);
 

@@ -56,6 +56,7 @@ SIGNATURES = {
     "trtt_b200_plan3d_status": (_I, [_vp, _vp]),
     "trtt_b200_plan3d_set_tiles": (_I, [_vp, _I, _I]),
     "trtt_b200_plan3d_factorized": (_I, [_vp]),
+    "trtt_b200_sweep_bounds_info": (_I, [_I, _L, _L, _L, _D, _I, _L, _L, _D, _D, _L, _dp, _dp, _lp]),
     "trtt_b200_plan3d_set_columns": (_I, [_vp, _I]),
     "trtt_b200_plan3d_groups": (_I, [_vp, _vp]),
     "trtt_b200_plan3d_wls_grad": (_I, [_vp, _vp, _vp, _vp, _vp, _vp, _vp]),

@@ -477,6 +477,28 @@ extern "C" int trtt_b200_plan3d_set_group_shape(trtt_b200_plan3d *pl, int band_r
   return 0;
 }
 
+extern "C" int trtt_b200_sweep_bounds_info(int geometry, long nx, long ny, long nz, double s_scl, int s_deg, long nu,
+                                           long nv, double u_scl, double v_scl, long nviews, const double *xos,
+                                           const double *xsd, long *info)
+{
+  clear_error();
+  const int geom = geom_code(geometry);
+  if (geom < 0) return fail("sweep_bounds_info: geometry must be PARALLEL_BEAM or CONE_BEAM");
+  if (!xos || !xsd || !info) return fail("sweep_bounds_info: null argument");
+  if (const char *why = check_sizes3d(nx, ny, nz, nu, nv, nviews)) return fail(std::string("sweep_bounds_info: ") + why);
+  const Params3D P = make_params(geom, nx, ny, nz, s_scl, s_deg, nullptr, 0, 1.0, 0.0, nu, nv, u_scl, v_scl);
+  std::vector<View3D> views(nviews);
+  bool fact = true;
+  for (long v = 0; v < nviews; ++v) {
+    make_view3d(P, xos + 12 * v, xsd + 12 * v, views[v]);
+    fact = fact && views[v].factorized;
+  }
+  const SweepBounds b = fact ? sweep_bounds(P, views.data(), nviews) : SweepBounds{};
+  const long out[5] = {b.rows, b.u0, b.u1, b.v0, b.v1};
+  std::copy(out, out + 5, info);
+  return 0;
+}
+
 extern "C" int trtt_b200_plan3d_factorized(const trtt_b200_plan3d *pl)
 {
   return pl && pl->factorized ? 1 : 0;

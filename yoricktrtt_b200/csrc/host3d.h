@@ -222,12 +222,15 @@ inline void choose_band(int nu, int nv, int &band_rows, int &warps)
   band_rows = rows >= 2 ? (int)rows : 0;
 }
 
-// Bounds for the sweep and gather kernels over the factorised views of a closed-form plan:
+// Bounds for the sweep and gather kernels over the factorised views of a plan:
 // the detector rows of one voxel column's v footprint, and the part of the
 // detector that any footprint can reach (a volume's shadow seldom fills the
-// detector; the tiles cover no more than it).  rows = 0 where the kernel does
-// not apply: a footprint that is not the cubic's 4 voxels wide (a walk
-// starts at a zero of the primitive), a source within the volume.
+// detector; the tiles cover no more than it).  Positions are quotients of affine
+// functions of the voxel, so the grid's corners bound them as long as neither
+// denominator changes sign over the grid.  rows = 0 where the kernels do
+// not apply: a closed-form footprint that is not the cubic's 4 voxels wide (a
+// walk starts at a zero of the primitive), a source within the volume, a tilted
+// detector whose plane through the source crosses the volume.
 inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nviews)
 {
   SweepBounds b;
@@ -263,7 +266,8 @@ inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nvi
       v1 = std::fmax(v1, v);
     }
     if (P.geom == GEOM_CONE) {
-      if (!(wmin * wmax > 0.0) || (P.model == MODEL_TABLE && dneg % 8 != 0)) return b;
+      // a pole of u and v inside the grid: the corners bound nothing
+      if (!(wmin * wmax > 0.0) || dneg % 8 != 0) return b;
       // nearest corner: largest magnification; outermost: largest obliquity
       const double magn = std::fabs(V.a4m) / std::fmin(std::fabs(wmin), std::fabs(wmax));
       hsv = std::fmax(hsv, P.hs0 * P.h_v0 * magn * std::sqrt(1.0 + dv2));
