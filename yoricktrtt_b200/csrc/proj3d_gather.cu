@@ -52,7 +52,7 @@ struct GatherCol {
 };
 
 // Shared memory of one warp: records, weight table, four profile rows of
-// `cap` cells with zeros before and after them.
+// `cap` cells with zeros before and after them, a GatherRest.
 __host__ __device__ constexpr size_t gather_row(int cap) { return (size_t)((cap + 2 * kSweepGuard + 3) & ~3); }
 template <int MODEL> struct GatherRec {
   using T = GatherCol;
@@ -66,7 +66,8 @@ template <> struct GatherRec<MODEL_TABLE> {
 };
 template <int MODEL> __host__ __device__ constexpr size_t gather_warp_bytes(int cap)
 {
-  return GatherRec<MODEL>::batch * kNC * sizeof(typename GatherRec<MODEL>::T) + sizeof(float2) * kTabRows * kNC + sizeof(float) * kNC * gather_row(cap);
+  return GatherRec<MODEL>::batch * kNC * sizeof(typename GatherRec<MODEL>::T) + sizeof(float2) * kTabRows * kNC + sizeof(float) * kNC * gather_row(cap) +
+         32;
 }
 
 template <int GEOM>
@@ -142,9 +143,80 @@ __device__ __forceinline__ void kahan(float &acc, float &cmp, float term)
   acc = t;
 }
 
+// What a warp with a sum that is not finite has left: the sums of the gates g[0]
+// and g[1] from the views start[0] and start[1] (in the order taken) on, and all
+// from view `next` on.
+struct GatherRest {
+  int start[2], g[2], next;
+};
+
+// The terms that a warp has left, each over its voxel's own rows and cells alone,
+// into the volume.  (A column's profile takes its neighbours' rows with weights of
+// 0, and a walk the cells of the voxel beside its own: one detector cell there that
+// is not finite spoils a voxel's sum.)  Voxel by voxel and view by view in FP64
+// sums, far slower than the kernel, after the kernel's loops, so that nothing of it
+// is alive in them (marked and mended view by view it cost 3 to 4% of every
+// transpose, here 0 to 2.6%); no call with finite data comes here.
+template <int GEOM, int PP, bool GATED, int MODEL>
+__device__ __noinline__ void gather_rest(const GatherLaunch &A, const GatherRest &R, int i, int j, int pb, int first,
+                                         int step)
+{
+  const Params3D &P = A.P;
+  const int lig = threadIdx.x & (kH - 1), nview = A.order ? A.norder : A.view_hi - A.view_lo;
+  if (i >= P.nx) return;
+  for (int e = 0; e < 2 * PP; ++e) {
+    const int k = 2 * pb + (MODEL == MODEL_TABLE ? lig + kH * e : 2 * (lig + kH * (e >> 1)) + (e & 1));
+    if (k >= P.nz) continue;
+    float *dst = A.vol + ((long)j * P.nx + i) * P.nz + k;
+    double sum[2] = {0.0, 0.0};
+    int g[2] = {GATED ? -1 : 0, -1};
+    for (int n = first; n < nview; ++n) {
+      if ((n - first) % step >= GatherRec<MODEL>::batch) continue;  // another warp's batch
+      const int view = A.order ? A.order[n] : A.view_lo + n;
+      if (view < A.view_lo || view >= A.view_hi) continue;
+      const View3D &V = A.views[view];
+      ColGeo<MODEL> c;
+      typename AxisOf<MODEL>::type ax;
+      float rho, s = 0.f;
+      column_geo<GEOM, MODEL>(P, V, i, j, 0, c);
+      if (c.bad || c.vax.n <= 0 || !voxel_u<GEOM, MODEL>(P, V, c, k, ax, rho)) continue;
+      const float *img = A.sino + (long)(view - A.view_lo) * A.sino_view_stride + (long)c.vax.lo * P.nu + ax.lo;
+      for (int l = 0; l < ax.n; ++l) {
+        const float w = axis_weight<MODEL>(ax, l, P);
+        if (w == 0.f) continue;
+        float q = 0.f;
+        for (int m = 0; m < c.vax.n; ++m) {
+          const float wv = axis_weight<MODEL>(c.vax, m, P);
+          if (wv != 0.f) q = fmaf(wv, __ldg(img + (long)m * P.nu + l), q);
+        }
+        s = fmaf(w, q, s);
+      }
+      if (!GATED) {
+        sum[0] += (double)(rho * s);
+        continue;
+      }
+      const GatePair gp = A.pairs[view];
+      for (int h = 0; h < 2; ++h) {
+        const int to = h ? gp.g1 : gp.g0;
+        if (to < 0) continue;
+        if (n < R.next && !(to == R.g[0] && n >= R.start[0]) && !(to == R.g[1] && n >= R.start[1])) continue;
+        const int a = to == g[0] ? 0 : (to == g[1] ? 1 : h);
+        if (to != g[a]) {
+          if (g[a] >= 0) dst[(long)g[a] * A.gate_stride] += (float)sum[a];
+          g[a] = to;
+          sum[a] = 0.0;
+        }
+        sum[a] += (double)((h ? gp.w1 : gp.w0) * (rho * s));
+      }
+    }
+    for (int a = 0; a < 2; ++a)  // (ungated: other warps may add to the voxel)
+      if (g[a] >= 0) atomicAdd(dst + (long)g[a] * A.gate_stride, (float)sum[a]);
+  }
+}
+
 template <int GEOM, int PP, bool GATED, int MODEL>
 __global__ void __launch_bounds__(32 * GatherRec<MODEL>::warps, MODEL == MODEL_TABLE ? 1 : (GATED || PP > 3 ? 2 : 3))
-k_back3d_gather(const GatherLaunch A)
+k_back3d_gather(const __grid_constant__ GatherLaunch A)
 {
   extern __shared__ __align__(16) unsigned char smem_all[];
   using Rec = typename GatherRec<MODEL>::T;
@@ -172,6 +244,7 @@ k_back3d_gather(const GatherLaunch A)
   Rec *recs = reinterpret_cast<Rec *>(smem + warp * wb);
   float2 *wtab = reinterpret_cast<float2 *>(recs + kBatch * kNC);
   float *Q = reinterpret_cast<float *>(wtab + kTabRows * kNC);
+  GatherRest &rest = *reinterpret_cast<GatherRest *>(Q + kNC * qrow);
   for (int t = lane; t < kNC * qrow; t += 32) Q[t] = 0.f;
   __syncwarp();
   float acc[NA][PP][2], cmp[NA][PP][2];
@@ -206,9 +279,20 @@ k_back3d_gather(const GatherLaunch A)
         cmp[a][i][e] = 0.f;
       }
   };
+  // some sum of the warp is not finite
+  auto spoiled = [&]() {
+    float m = 0.f;
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+#pragma unroll
+      for (int i = 0; i < PP; ++i) m += fabsf(acc[a][i][0]) + fabsf(acc[a][i][1]);
+    return __any_sync(FULLM, !is_finite(m));
+  };
+  bool left = false;
+  if (GATED) rest = GatherRest{{0, 0}, {-1, -1}, INT_MAX};
   const int nview = active ? (A.order ? A.norder : A.view_hi - A.view_lo) : 0;
   const int vstep = kBatch * A.vsplit;
-  for (int vb = vs * kBatch; vb < nview; vb += vstep) {
+  for (int vb = vs * kBatch; vb < nview && !left; vb += vstep) {
     // ---- records of kBatch views x kNC columns ---------------------------
     {
       const int n = vb + lane / kNC, ci = i0 + lane % kNC;
@@ -252,6 +336,11 @@ k_back3d_gather(const GatherLaunch A)
         wbv = gp.w1;
         two = gp.g1 >= 0;
         if (gp.g0 != ga || (gp.g1 >= 0 && gp.g1 != gb)) {
+          if (spoiled()) {
+            left = true;
+            rest.next = vb + b;
+            break;
+          }
           if (gp.g0 == gb) {  // the second gate becomes the first
             flush(0, ga);
 #pragma unroll
@@ -267,8 +356,13 @@ k_back3d_gather(const GatherLaunch A)
             if (gp.g0 != ga) flush(0, ga);
             flush(NA - 1, gb);
           }
+          // (slot 1 starts anew in every case; a gate that moves to slot 0 keeps its start)
+          if (gp.g0 != ga) rest.start[0] = gp.g0 == gb ? rest.start[1] : vb + b;
+          rest.start[1] = vb + b;
           ga = gp.g0;
           gb = gp.g1;
+          rest.g[0] = ga;
+          rest.g[1] = gb;
         }
       }
       // ---- v-collapsed profiles of the four columns ------------------------
@@ -507,39 +601,43 @@ k_back3d_gather(const GatherLaunch A)
       __syncwarp();
     }
   }
+  left = left || spoiled();
   if (GATED) {
-    flush(0, ga);
-    flush(NA - 1, gb);
-    return;
-  }
-  if (A.vsplit == 1) {
-    flush(0, 0);
-    return;
-  }
-  // the warps of a column group add up: sums and compensations to shared memory
-  __syncthreads();
-  float2 *part = reinterpret_cast<float2 *>(smem);
-#pragma unroll
-  for (int i = 0; i < PP; ++i)
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-      part[(2 * i + e) * (32 * kWarps) + threadIdx.x] = make_float2(acc[0][i][e], cmp[0][i][e]);
-  __syncthreads();
-  if (vs == 0) {
+    if (!left) {
+      flush(0, ga);
+      flush(NA - 1, gb);
+    }
+  } else if (A.vsplit == 1) {
+    if (!left) flush(0, 0);
+  } else {
+    // the warps of a column group add up: sums and compensations to shared memory
+    __syncthreads();
+    float2 *part = reinterpret_cast<float2 *>(smem);
 #pragma unroll
     for (int i = 0; i < PP; ++i)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        double s = 0.0;
-        for (int w = 0; w < A.vsplit; ++w) {
-          const float2 p = part[(2 * i + e) * (32 * kWarps) + threadIdx.x + 32 * w];
-          s += (double)p.x - (double)p.y;
+      for (int e = 0; e < 2; ++e)
+        part[(2 * i + e) * (32 * kWarps) + threadIdx.x] =
+            left ? f2(0.f) : make_float2(acc[0][i][e], cmp[0][i][e]);
+    __syncthreads();
+    if (vs == 0) {
+#pragma unroll
+      for (int i = 0; i < PP; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          double s = 0.0;
+          for (int w = 0; w < A.vsplit; ++w) {
+            const float2 p = part[(2 * i + e) * (32 * kWarps) + threadIdx.x + 32 * w];
+            s += (double)p.x - (double)p.y;
+          }
+          acc[0][i][e] = (float)s;
+          cmp[0][i][e] = 0.f;
         }
-        acc[0][i][e] = (float)s;
-        cmp[0][i][e] = 0.f;
-      }
-    flush(0, 0);
+      flush(0, 0);
+    }
+    __syncthreads();
   }
+  if (left && active) gather_rest<GEOM, PP, GATED, MODEL>(A, rest, col_i, j, pb, vs * kBatch, vstep);
 }
 
 template <int GEOM, int PP, int MODEL>

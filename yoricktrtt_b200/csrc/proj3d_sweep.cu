@@ -30,11 +30,11 @@ namespace {
 constexpr int kMaxSplit = 8;    // portable cluster size
 
 template <int GEOM, int G, int Q, int H, int WARPS, int MINB, int MODEL>
-__global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const SweepLaunch A)
+__global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const __grid_constant__ SweepLaunch A)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ View3D sV;
-  __shared__ int s_next;
+  __shared__ int s_next, s_odd;
   const Params3D &P = A.P;
   constexpr int US = 64 * Q;  // floats of a band row
   constexpr size_t WB = sweep_warp_bytes<G, Q, H, MODEL>();
@@ -61,16 +61,24 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const SweepLau
   if (threadIdx.x < (int)(sizeof(View3D) / 8))
     reinterpret_cast<double *>(&sV)[threadIdx.x] =
         reinterpret_cast<const double *>(A.views + (A.groups ? A.groups[4 * blockIdx.y] : (int)blockIdx.y))[threadIdx.x];
-  if (threadIdx.x == 0) s_next = 0;
+  if (threadIdx.x == 0) {
+    s_next = 0;
+    s_odd = 0;
+  }
   for (int t = threadIdx.x; t < rows * US; t += blockDim.x) band[t] = 0.f;
   for (int t = threadIdx.x; t < sweep_groups(R) * SweepStrip<Q, H>::NS; t += blockDim.x) locks[t] = 0;
   for (int t = threadIdx.x & 31; t < NC * (US + G * kSweepGuard) + G * kSweepGuard; t += 32) prof[t] = 0.f;
   __syncthreads();
   sweep_item<GEOM, G, Q, H, MODEL>(P, sV, A.vol, A.gate_stride, v0, v1, u0, u1, band, prof, recs, wtab, locks, &s_next,
-                                   rank, S, T, A.err);
+                                   rank, S, T, &s_odd, A.err);
+  __syncthreads();
+  if (s_odd) {
+    sweep_odd<GEOM, G, Q, H, MODEL>(P, sV, A.vol, A.gate_stride, T, v0, v1, u0, u1, band, locks, rank, S, A.err);
+    __syncthreads();
+  }
   const int nrow = v1 - v0, ncell = u1 - u0;
   cg::cluster_group cl = cg::this_cluster();
-  if (S == 1) __syncthreads(); else cl.sync();
+  if (S > 1) cl.sync();
   // the cluster's bands, added in rank order; each CTA writes its share
 #pragma unroll
   for (int m = 0; m < G; ++m) {

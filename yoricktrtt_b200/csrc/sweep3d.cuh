@@ -272,6 +272,8 @@ __device__ __forceinline__ bool sweep_record(const Params3D &P, const View3D &V,
   return true;
 }
 
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) < __int_as_float(0x7f800000); }
+
 // A lane's walk: `steps` double cells from cell `rel` of the row, voxels a and
 // c with abscissae ax and cx at the second edge and steps da, dc per cell.  CHECK: cells outside [0, ncell) are left alone (some
 // lane's walk leaves the row's guards).  All lanes of the warp take it.
@@ -314,7 +316,7 @@ __device__ __forceinline__ void sweep_walk(typename SweepVec<G>::T *row, int rel
 template <int GEOM, int G>
 __device__ __noinline__ void sweep_profile_any(const Params3D &P, const View3D &V, const float *__restrict__ vol,
                                                long gate_stride, int ci, int cj, int p0, int p1, int u0, int ncell,
-                                               float *prof)
+                                               float *prof, int *odd)
 {
   const int lane = threadIdx.x & 31;
   ColGeo<MODEL_CUBIC> c;
@@ -326,6 +328,10 @@ __device__ __noinline__ void sweep_profile_any(const Params3D &P, const View3D &
     for (int m = 0; m < G; ++m) {
       const float x = vox_val(vol, gate_stride, V, turned_col(ci, cj, 4 - sweep_turn<G>(m), P.nx, P.ny) * P.nz + k);
       if (x == 0.f) continue;
+      if (!is_finite(x)) {
+        *odd = 1;
+        continue;
+      }
       float Fp = F0;
       for (int l = 0; l < up.n0; ++l) {
         const float F = cubic_prim2(f2(fmaf((float)(l + 1), up.inc.x, up.start.x))).x;
@@ -366,7 +372,7 @@ __device__ __forceinline__ float gate_value(const View3D &V, const float *colp, 
 template <int GEOM, int H>
 __device__ __forceinline__ unsigned table_profiles(const Params3D &P, const View3D &V, const TableSh &T,
                                                    const TableCol &r, bool mine, int q, const float *colp, long dgate,
-                                                   bool gated, int u0, int u1, float *row)
+                                                   bool gated, int u0, int u1, float *row, int *odd)
 {
   const int lig = threadIdx.x & (H - 1);
   const int k0 = r.k0, k1 = mine ? r.k1 : k0, nk = __reduce_max_sync(FULLM, k1 - k0);
@@ -378,9 +384,13 @@ __device__ __forceinline__ unsigned table_profiles(const Params3D &P, const View
       sub = 0;
       pp += H * q;
     }
-    const float x = k < k1 ? gate_value(V, colp, dgate, gated, k) : 0.f;
+    float x = k < k1 ? gate_value(V, colp, dgate, gated, k) : 0.f;
     const unsigned some = __ballot_sync(FULLM, x != 0.f);
     if (!some) continue;
+    if (!is_finite(x)) {
+      *odd = 1;
+      x = 0.f;
+    }
     touched |= some;
     TableVox v;
     table_voxel<GEOM>(P, V, T, r, table_kc<GEOM>(V, k), u0, u1, v);
@@ -414,11 +424,16 @@ __device__ __forceinline__ unsigned table_profiles(const Params3D &P, const View
 // coincide on the detector.
 template <int GEOM>
 __device__ __noinline__ void table_profile_any(const Params3D &P, const View3D &V, const TableSh &T, const TableCol &r,
-                                               const float *colp, long dgate, bool gated, int u0, int u1, float *row)
+                                               const float *colp, long dgate, bool gated, int u0, int u1, float *row,
+                                               int *odd)
 {
   for (int k = r.k0 + (threadIdx.x & 31); k < r.k1; k += 32) {
     const float x = gate_value(V, colp, dgate, gated, k);
     if (x == 0.f) continue;
+    if (!is_finite(x)) {
+      *odd = 1;
+      continue;
+    }
     TableVox v;
     table_voxel<GEOM>(P, V, T, r, table_kc<GEOM>(V, k), u0, u1, v);
     for (int t = v.s; t < v.s + v.n; ++t) {
@@ -433,12 +448,13 @@ __device__ __noinline__ void table_profile_any(const Params3D &P, const View3D &
 // All threads of the CTA call it; band, prof (this warp's profile rows) and
 // locks are zero on entry, prof zero on exit; no final barrier.  `next`: the
 // CTA's line counter (0 on entry); the CTA takes lines rank, rank + split, ...
-// The tile has u1 - u0 <= 64 Q / G cells.
+// The tile has u1 - u0 <= 64 Q / G cells.  *odd (0 on entry) is set where a voxel
+// is not finite; such voxels are left out, for sweep_odd.
 template <int GEOM, int G, int Q, int H, int MODEL>
 __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, const float *__restrict__ vol,
                                            long gate_stride, int v0, int v1, int u0, int u1, float *band, float *prof,
                                            typename SweepRec<MODEL>::T *recs, float2 *wtab, int *locks, int *next,
-                                           int rank, int split, const TableSh &T, int *__restrict__ err)
+                                           int rank, int split, const TableSh &T, int *odd, int *__restrict__ err)
 {
   using Rec = typename SweepRec<MODEL>::T;
   constexpr int RB = SweepRec<MODEL>::batch;
@@ -490,12 +506,12 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
           if (!__any_sync(FULLM, r.q_lanes == 0)) {
             const float *colp = volg + turned_col(S.axis ? ln : r.col, S.axis ? r.col : ln, 0, nx, ny) * nz;
             touched = table_profiles<GEOM, H>(P, V, T, r, mine, __reduce_max_sync(FULLM, r.q_lanes), colp, dgate,
-                                              gated, u0, u1, prof + kSweepGuard + grp * PS);
+                                              gated, u0, u1, prof + kSweepGuard + grp * PS, odd);
           } else {
             for (int g = 0; g < NC && b + g < cnt; ++g) {
               const Rec &o = recs[b + g];
               const float *colp = volg + turned_col(S.axis ? ln : o.col, S.axis ? o.col : ln, 0, nx, ny) * nz;
-              table_profile_any<GEOM>(P, V, T, o, colp, dgate, gated, u0, u1, prof + kSweepGuard + g * PS);
+              table_profile_any<GEOM>(P, V, T, o, colp, dgate, gated, u0, u1, prof + kSweepGuard + g * PS, odd);
             }
             touched = FULLM;
             __syncwarp();
@@ -538,7 +554,7 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
             const int ke = 2 * p, ko = ke + 1;
             const bool ine = p < p1 && ke < nz, ino = p < p1 && ko < nz;
             float xe[G], xo[G];
-            bool any = false;
+            float mag = 0.f;  // of the values together: 0 only if all are, infinite or NaN if one is
 #pragma unroll
             for (int m = 0; m < G; ++m) {
               xe[m] = ine ? __ldg(colp[m] + ke) : 0.f;
@@ -552,10 +568,18 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
                   xo[m] *= V.w0;
                 }
               }
-              any = any || xe[m] != 0.f || xo[m] != 0.f;
+              mag += fabsf(xe[m]) + fabsf(xo[m]);
             }
-            const unsigned some = __ballot_sync(FULLM, any);
+            const unsigned some = __ballot_sync(FULLM, mag != 0.f);
             if (!some) continue;
+            if (__any_sync(FULLM, !is_finite(mag))) {  // left to sweep_odd
+              *odd = 1;
+#pragma unroll
+              for (int m = 0; m < G; ++m) {
+                if (!is_finite(xe[m])) xe[m] = 0.f;
+                if (!is_finite(xo[m])) xo[m] = 0.f;
+              }
+            }
             touched |= some;
             const long long uo = ue0 + B, ua = up ? ue0 : uo, uc = up ? uo : ue0;
             const int Ia = (int)(ua >> 32), Ic = (int)(uc >> 32);
@@ -601,7 +625,7 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
           for (int g = 0; g < NC && b + g < cnt; ++g) {
             const Rec &o = recs[b + g];
             sweep_profile_any<GEOM, G>(P, V, vol, gate_stride, S.axis ? ln : o.col, S.axis ? o.col : ln, o.p0, o.p1,
-                                    u0, ncell, prof + G * (kSweepGuard + g * PS));
+                                       u0, ncell, prof + G * (kSweepGuard + g * PS), odd);
           }
           touched = FULLM;
           __syncwarp();
@@ -674,6 +698,109 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
           }
           __syncwarp();
         }
+      }
+    }
+  }
+}
+
+// The voxels that are not finite, which sweep_item leaves out: each is added to the
+// cells and rows where its own weights are not zero.  (The sums of sweep_item over
+// several columns and voxels take products with weights of 0, harmless as long as
+// every factor is finite.)  Voxel by voxel, the whole warp over the cells, under
+// the band's locks.  A second pass over the CTA's lines, so that nothing of it is
+// alive in the loops of the first (called from there it cost 4 to 7% of every
+// projection; the test of the values that is left there 0 to 1.5%); no call with a
+// finite volume comes here.  All threads of the CTA call it after a barrier.
+template <int GEOM, int G, int Q, int H, int MODEL>
+__device__ __noinline__ void sweep_odd(const Params3D &P, const View3D &V, const float *__restrict__ vol,
+                                       long gate_stride, const TableSh &T, int v0, int v1, int u0, int u1, float *band,
+                                       int *locks, int rank, int split, int *__restrict__ err)
+{
+  using Strip = SweepStrip<Q, H>;
+  constexpr int SP = Strip::SP, NS = Strip::NS;
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  SweepView S;
+  sweep_view<GEOM>(P, V, S);
+  const int n = S.axis ? P.ny : P.nx, nl = S.axis ? P.nx : P.ny;
+  for (int unit = threadIdx.x >> 5; (unit / n) * split + rank < nl; unit += warps) {
+    const int ln = (unit / n) * split + rank, a = unit % n;  // the lines that the CTA took in the first pass
+    const int ci = S.axis ? ln : a, cj = S.axis ? a : ln;
+    typename SweepRec<MODEL>::T o;
+    if (!sweep_record<GEOM>(P, V, ci, cj, v0, v1, u0, u1, o, err)) continue;
+    ColGeo<MODEL_CUBIC> c;
+    int ka, kb;
+    if constexpr (MODEL == MODEL_TABLE) {
+      ka = o.k0;
+      kb = o.k1;
+    } else {
+      column_geo<GEOM, MODEL_CUBIC>(P, V, ci, cj, 0, c);
+      ka = 2 * o.p0;
+      kb = min(2 * o.p1, P.nz);
+    }
+    const int r0 = max(o.lo, v0), r1 = min(o.lo + o.n, v1);
+    for (int k0 = ka; k0 < kb; k0 += 32) {
+      float mine[G];
+      bool bad = false;
+      for (int m = 0; m < G; ++m) {
+        const long col = turned_col(ci, cj, 4 - sweep_turn<G>(m), P.nx, P.ny);
+        mine[m] = k0 + lane < kb ? vox_val(vol, gate_stride, V, col * P.nz + k0 + lane) : 0.f;
+        bad = bad || !is_finite(mine[m]);
+      }
+      for (unsigned left = __ballot_sync(FULLM, bad); left; left &= left - 1) {
+        const int src = __ffs(left) - 1, k = k0 + src;
+        float x[G];
+        for (int m = 0; m < G; ++m) x[m] = __shfl_sync(FULLM, mine[m], src);
+        UPair up;
+        TableVox t;
+        int f, nf;  // cells [f, f + nf)
+        float rho;
+        if constexpr (MODEL == MODEL_TABLE) {
+          table_voxel<GEOM>(P, V, T, o, table_kc<GEOM>(V, k), u0, u1, t);
+          f = t.f + t.s;
+          nf = t.n;
+          rho = t.rho;
+        } else {
+          voxel_u_pair<GEOM>(P, V, c, k, k, up);
+          f = up.lo0;
+          nf = up.n0;
+          rho = up.rho.x;
+        }
+        for (int gr = (r0 - v0) / kSweepRows; gr < sweep_groups(r1 - v0); ++gr)
+          for (int s = 0; s < NS; ++s) {
+            int *lock = locks + gr * NS + s;
+            if (!row_lock(lock, err)) continue;
+            for (int q = 0; q < 2 * SP; ++q) {
+              // float q of the lane's pairs: a member of a cell
+              const int at = 2 * (lane + 32 * (s * SP + (q >> 1))) + (q & 1), u = u0 + at / G, l = u - f;
+              if (l < 0 || l >= nf || u >= u1) continue;
+              float w;
+              if constexpr (MODEL == MODEL_TABLE) {
+                const double e = (double)(u - t.f - t.l0);
+                w = (float)(table_at(T, dadd(t.start, dmul(e + 1.0, t.inc))) -
+                            table_at(T, dadd(t.start, dmul(e, t.inc))));
+              } else {
+                const float a = l == 0 ? first_edge_prim2(up).x : cubic_prim2(f2(fmaf((float)l, up.inc.x, up.start.x))).x;
+                w = cubic_prim2(f2(fmaf((float)(l + 1), up.inc.x, up.start.x))).x - a;
+              }
+              float xm = 0.f;
+              for (int m = 0; m < G; ++m)
+                if (at % G == m) xm = x[m];
+              if (w == 0.f || is_finite(xm)) continue;
+              for (int r = max(r0, v0 + gr * kSweepRows); r < min(r1, v0 + (gr + 1) * kSweepRows); ++r) {
+                float wv;
+                if constexpr (MODEL == MODEL_TABLE) {
+                  wv = table_weight_v(T, o, r - o.lo);
+                } else {
+                  AxisCubic ax;
+                  ax.start = o.vstart;
+                  ax.inc = o.vinc;
+                  wv = edge_cubic(ax, r - o.lo + 1) - edge_cubic(ax, r - o.lo);
+                }
+                if (wv != 0.f) band[(size_t)(r - v0) * (64 * Q) + at] += wv * (w * (xm * rho));
+              }
+            }
+            row_unlock(lock);
+          }
       }
     }
   }
