@@ -398,19 +398,28 @@ extern "C" int trtt_b200_plan3d_wls_grad(trtt_b200_plan3d *pl, const float *vol,
     return fail("plan3d_wls_grad: needs the closed-form model and column-factorised views");
   cudaStream_t st = (cudaStream_t)stream;
   const Params3D &P = pl->P;
-  if (!pl->wls_set && pl->wls_extra == 0 && pl->band_rows > 0 && pl->nviews <= 65535) {
+  int rows = 0, warps = 16;
+  choose_band(P.nu, P.nv, rows, warps);
+  if (!pl->wls_set && pl->wls_extra == 0 && rows > 0 && pl->nviews <= 65535) {
     // direct projection, residual with its cost, transpose: three launches, each
     // at its own shape.  10 gates of 128 x 128 x 64, 347 views on 256^2: 20.5 ms;
     // the persistent launch 26.0 at its best shape and 28.5-33 at its default
     // one.  The direct projection is the band kernel, whose FP32 sums are the
     // persistent launch's: the FP64 cost shows their rounding (8e-8 below the
-    // exact value), and callers compare costs to 1e-9.
+    // exact value), and callers compare costs to 1e-9.  What set_tiles chose for
+    // plan3d_forward does not count here, as it does not in the persistent launch
+    // (the tensor-core band's sums are 1.5e-5 off).
     const long npix = (long)P.nu * P.nv;
     TRTT_CK(pl->resid.ensure(sizeof(float) * (size_t)pl->nviews * npix));
     float *resid = pl->resid.as<float>();
     TRTT_CK(cudaMemsetAsync(resid, 0, sizeof(float) * (size_t)pl->nviews * npix, st));
     TRTT_CK(cudaMemsetAsync(cost, 0, sizeof(double), st));
-    TRTT_CK(launch_fwd3d(fwd_launch(pl, vol, resid, 0, pl->nviews), st));
+    Fwd3DLaunch F = fwd_launch(pl, vol, resid, 0, pl->nviews);
+    F.band_rows = rows;
+    F.warps = warps;
+    F.pull = F.tc = 0;
+    F.cols = 1;
+    TRTT_CK(launch_fwd3d(F, st));
     TRTT_CK(launch_wls_residual(resid, y, w, pl->nviews * npix, cost, st));
     TRTT_CK(launch_back3d(back_launch(pl, resid, grad, 0, pl->nviews), st));
     count_launch(3);
