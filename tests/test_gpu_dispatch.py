@@ -1,0 +1,56 @@
+"""Which kernels a plan launches after a shape was asked for, refused or given
+back (names from the CUDA activity record)."""
+import numpy as np
+import pytest
+
+from yoricktrtt_b200 import geometry as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(views=5, theta=True, n=24, nz=16):
+    from yoricktrtt_b200.projectors import Projector3D
+    th = np.linspace(0.1, 6.0, views) ** 1.01 if theta else None
+    return Projector3D(G.circular_scan_3d(n, n, nz, 1.0, 3, 40, 44, 1.0, 1.0, views, rsc=100.0, rsd=150.0, theta=th))
+
+
+def _kernels(fn):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    fn()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+        fn()
+        torch.cuda.synchronize()
+    names = " ".join(e.key for e in p.key_averages())
+    if "k_" not in names:
+        pytest.skip("no CUDA activity record")
+    return names
+
+
+def _forward(pr):
+    import torch
+    vol = torch.ones(pr.volume_shape(), device="cuda")
+    return _kernels(lambda: pr.forward(vol))
+
+
+@pytest.mark.parametrize("tiles", [(16, 99), (16, 1), (100000, 0), (100000, 8)])
+def test_refused_tiles_leave_the_default_kernel(tiles):
+    from yoricktrtt_b200 import _lib
+    pr = _plan()
+    assert "k_fwd3d_sweep" in _forward(pr)
+    assert _lib.load().trtt_b200_plan3d_set_tiles(pr._h, *tiles) == -1
+    assert "k_fwd3d_sweep" in _forward(pr)
+
+
+def test_refused_tiles_leave_the_shape_asked_for():
+    from yoricktrtt_b200 import _lib
+    pr = _plan()
+    pr.set_tiles(-2, 0)
+    assert "k_fwd3d_pull" in _forward(pr)
+    assert _lib.load().trtt_b200_plan3d_set_tiles(pr._h, 16, 99) == -1
+    assert "k_fwd3d_pull" in _forward(pr)
+    pr.set_tiles(16, 8)
+    assert "k_fwd3d_band" in _forward(pr)
+    pr.set_tiles(0, 0)
+    assert "k_fwd3d_sweep" in _forward(pr)

@@ -273,16 +273,18 @@ extern "C" int trtt_b200_plan3d_set_tiles(trtt_b200_plan3d *pl, int band_rows, i
 {
   clear_error();
   if (!pl) return fail("plan3d_set_tiles: null plan");
-  pl->tiles_set = !(band_rows == 0 && warps == 0);
+  // (a request that is refused leaves the plan as it was)
   if (band_rows == 0 && warps == 0) {  // defaults
     pl->pull = 0;
     pl->tc = 0;
     choose_band(pl->P.nu, pl->P.nv, pl->band_rows, pl->warps);
+    pl->tiles_set = false;
     return 0;
   }
   if (band_rows == TRTT_B200_TILES_PULL) {  // atomic-free band kernel
     pl->pull = 1;
     pl->tc = 0;
+    pl->tiles_set = true;
     return 0;
   }
   if (band_rows == TRTT_B200_TILES_TENSOR) {  // tensor-core band kernel
@@ -291,21 +293,19 @@ extern "C" int trtt_b200_plan3d_set_tiles(trtt_b200_plan3d *pl, int band_rows, i
     pl->pull = 0;
     pl->tc = 1;
     if (pl->band_rows <= 0) choose_band(pl->P.nu, pl->P.nv, pl->band_rows, pl->warps);
+    pl->tiles_set = true;
     return 0;
   }
+  if (warps > 0 && (warps < 2 || warps > 16)) return fail("plan3d_set_tiles: warps must be in [2, 16]");
+  const int w = warps > 0 ? warps : pl->warps;
+  if (band_rows > 0 && (long)band_fast_smem(pl->P.nu, band_rows, w) > 227L * 1024)
+    return fail("plan3d_set_tiles: band does not fit in shared memory");
   pl->pull = 0;
   pl->tc = 0;
-  if (warps > 0) {
-    if (warps < 2 || warps > 16) return fail("plan3d_set_tiles: warps must be in [2, 16]");
-    pl->warps = warps;
-  }
-  if (band_rows < 0) {
-    pl->band_rows = 0;
-  } else if (band_rows > 0) {
-    const long smem = (long)band_fast_smem(pl->P.nu, band_rows, pl->warps);
-    if (smem > 227L * 1024) return fail("plan3d_set_tiles: band does not fit in shared memory");
-    pl->band_rows = band_rows > pl->P.nv ? pl->P.nv : band_rows;
-  }
+  pl->warps = w;
+  if (band_rows < 0) pl->band_rows = 0;
+  if (band_rows > 0) pl->band_rows = band_rows > pl->P.nv ? pl->P.nv : band_rows;
+  pl->tiles_set = true;
   return 0;
 }
 
