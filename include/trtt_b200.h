@@ -301,7 +301,10 @@ int trtt_b200_plan3d_set_group_tiles(trtt_b200_plan3d *plan, int band_rows4, int
  * detector cells per u tile (0: up to 256; else 32..256) and CTAs per SM
  * (1: one CTA of 22 warps, or 16 where 22 warps' profiles do not fit in
  * shared memory; 2: two CTAs of 16 warps, 64 registers per thread; 0
- * keeps).  -1 if the CTA's shared memory does not fit at that occupancy. */
+ * keeps).  -1 if the CTA's shared memory does not fit at that occupancy.
+ * A shape given here, or band rows given to set_group_tiles, selects that kernel
+ * (k_fwd3d_group) for the direct projection; all 0 here returns to the default,
+ * the sweep kernel. */
 int trtt_b200_plan3d_set_group_shape(trtt_b200_plan3d *plan, int band_rows4, int utile4,
                                      int ctas_per_sm4);
 

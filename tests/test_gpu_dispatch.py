@@ -54,3 +54,16 @@ def test_refused_tiles_leave_the_shape_asked_for():
     assert "k_fwd3d_band" in _forward(pr)
     pr.set_tiles(0, 0)
     assert "k_fwd3d_sweep" in _forward(pr)
+
+
+@pytest.mark.parametrize("ask", [lambda pr: pr.set_group_shape(16, 32, 2), lambda pr: pr.set_group_tiles(band_rows4=8)])
+def test_group_shape_can_be_given_back(ask):
+    pr = _plan(views=8, theta=False)
+    assert pr.groups() == (0, 0, 2)
+    assert "k_fwd3d_sweep" in _forward(pr)
+    ask(pr)
+    assert "k_fwd3d_group" in _forward(pr)
+    pr.set_group_tiles(back_chunk_bytes=1 << 20)  # no shape of the direct kernel
+    assert "k_fwd3d_group" in _forward(pr)
+    pr.set_group_shape()
+    assert "k_fwd3d_sweep" in _forward(pr)

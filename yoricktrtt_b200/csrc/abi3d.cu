@@ -479,7 +479,7 @@ extern "C" int trtt_b200_plan3d_set_group_shape(trtt_b200_plan3d *pl, int band_r
   const size_t smem = group_fwd_smem(4, rows, ut, group_fwd_warps(4, rows, ut, cpsm));
   if (smem > (cpsm == 2 ? 113u : 227u) * 1024u)
     return fail("plan3d_set_group_shape: the quad band does not fit in shared memory at that occupancy");
-  if (band_rows4 || utile4 || ctas_per_sm4) pl->group_set = true;
+  pl->group_set = band_rows4 || utile4 || ctas_per_sm4;
   if (band_rows4) pl->gband[2] = band_rows4;
   pl->gutile4 = utile4;
   if (ctas_per_sm4) pl->gminb4 = ctas_per_sm4;

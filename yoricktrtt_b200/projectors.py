@@ -115,7 +115,8 @@ class Projector3D:
 
     def set_group_shape(self, band_rows4=0, utile4=0, ctas_per_sm4=0):
         """Direct kernel shape for groups of 4 views (see
-        trtt_b200_plan3d_set_group_shape)."""
+        trtt_b200_plan3d_set_group_shape); no arguments: back to the default
+        kernel."""
         _lib.check(_lib.load().trtt_b200_plan3d_set_group_shape(self._h, band_rows4, utile4, ctas_per_sm4),
                    "trtt_b200_plan3d_set_group_shape")
 
