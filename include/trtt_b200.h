@@ -255,7 +255,8 @@ int trtt_b200_plan3d_wls_grad(trtt_b200_plan3d *plan, const float *vol, const fl
  * default), CTAs per SM (1: up to 128 registers per thread, 2: 64; 0
  * keeps), the bound of the device wait in seconds (0 keeps; 2 s by
  * default) and extra_wait, a test hook: column items also wait for
- * extra_wait band items that do not exist, so the bounded wait runs out. */
+ * extra_wait band items that do not exist, so the bounded wait runs out.
+ * All 0: back to the three launches. */
 int trtt_b200_plan3d_set_persistent(trtt_b200_plan3d *plan, int band_rows, int ctas_per_sm,
                                     double wait_seconds, int extra_wait);
 

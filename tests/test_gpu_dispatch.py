@@ -67,3 +67,22 @@ def test_group_shape_can_be_given_back(ask):
     assert "k_fwd3d_group" in _forward(pr)
     pr.set_group_shape()
     assert "k_fwd3d_sweep" in _forward(pr)
+
+
+def test_persistent_shape_can_be_given_back():
+    import torch
+    pr = _plan()
+    x = torch.rand(pr.volume_shape("columns"), device="cuda")
+    y = torch.rand(pr.detector_shape(), device="cuda")
+    grad = torch.zeros_like(x)
+    names = lambda: _kernels(lambda: pr.wls_grad(x, y, grad))
+    assert "k_wls_persistent" not in names()
+    pr.set_persistent(16, 1)
+    assert "k_wls_persistent" in names()
+    pr.set_persistent(wait_seconds=1.0)
+    assert "k_wls_persistent" in names()
+    pr.set_persistent()
+    assert "k_wls_persistent" not in names()
+    times, choice = pr.autotune_wls(x, y, reps=1)
+    assert (0, 0) in times and (16, 1) in times
+    assert ("k_wls_persistent" in names()) == (choice != (0, 0))

@@ -383,7 +383,10 @@ extern "C" int trtt_b200_plan3d_set_persistent(trtt_b200_plan3d *pl, int band_ro
     pl->wls_rows = band_rows;
   }
   if (ctas_per_sm) pl->wls_ctas = ctas_per_sm;
-  if (band_rows || ctas_per_sm) pl->wls_set = true;
+  if (band_rows || ctas_per_sm)
+    pl->wls_set = true;
+  else if (wait_seconds == 0.0 && extra_wait == 0)
+    pl->wls_set = false;
   if (wait_seconds > 0.0) pl->wls_wait_ns = (long long)(wait_seconds * 1e9);
   pl->wls_extra = extra_wait;
   return 0;
@@ -402,13 +405,13 @@ extern "C" int trtt_b200_plan3d_wls_grad(trtt_b200_plan3d *pl, const float *vol,
   choose_band(P.nu, P.nv, rows, warps);
   if (!pl->wls_set && pl->wls_extra == 0 && rows > 0 && pl->nviews <= 65535) {
     // direct projection, residual with its cost, transpose: three launches, each
-    // at its own shape.  10 gates of 128 x 128 x 64, 347 views on 256^2: 20.5 ms;
-    // the persistent launch 26.0 at its best shape and 28.5-33 at its default
-    // one.  The direct projection is the band kernel, whose FP32 sums are the
-    // persistent launch's: the FP64 cost shows their rounding (8e-8 below the
-    // exact value), and callers compare costs to 1e-9.  What set_tiles chose for
-    // plan3d_forward does not count here, as it does not in the persistent launch
-    // (the tensor-core band's sums are 1.5e-5 off).
+    // at its own shape.  10 gates of 128 x 128 x 64 on 256^2: 452 views of dense
+    // gates 20.6 ms, the persistent launch 26.0 at its best shape and 33.1 at its
+    // own default; 347 views of a phantom 12.7 ms, 16.3 and 20.3.  The direct
+    // projection is the band kernel, so that both forms form the cost of the same
+    // FP32 sums (8e-8 below FP64; the sweep kernel's are 2.5e-8 from them).  What
+    // set_tiles chose for plan3d_forward does not count here, as it does not in the
+    // persistent launch (the tensor-core band's sums are 1.5e-5 off).
     const long npix = (long)P.nu * P.nv;
     TRTT_CK(pl->resid.ensure(sizeof(float) * (size_t)pl->nviews * npix));
     float *resid = pl->resid.as<float>();

@@ -146,16 +146,20 @@ class Projector3D:
         return cost
 
     def set_persistent(self, band_rows=0, ctas_per_sm=0, wait_seconds=0.0, extra_wait=0):
+        """Persistent launch for wls_grad with this shape (see
+        trtt_b200_plan3d_set_persistent); no arguments: back to the three
+        launches of the default."""
         _lib.check(_lib.load().trtt_b200_plan3d_set_persistent(
             self._h, band_rows, ctas_per_sm, float(wait_seconds), extra_wait),
             "trtt_b200_plan3d_set_persistent")
 
-    WLS_CANDIDATES = [(16, 1), (32, 1), (16, 2), (32, 2), (8, 2)]
+    WLS_CANDIDATES = [(0, 0), (16, 1), (32, 1), (16, 2), (32, 2), (8, 2)]
 
     def autotune_wls(self, vol, y, w=None, candidates=None, reps=2):
-        """Time the persistent launch with each (band rows, CTAs per SM)
-        candidate on the given data and keep the fastest; returns
-        ({candidate: ms}, choice)."""
+        """Time wls_grad on the given data with each (band rows, CTAs per SM)
+        shape of the persistent launch and with the three launches of the
+        default, (0, 0), and keep the fastest; returns ({candidate: ms},
+        choice)."""
         torch = _torch()
         grad = torch.zeros_like(vol)
         times = {}

@@ -174,10 +174,10 @@ def cone3d_recon(maxiter=100, frtol=1e-6, seed=0, n=256, nd=512, views=360):
 def gates4d(nt=10, seed=0, replays=5):
     """10 gates of 128x128x64 (breathing phantom), views per gate from
     U{20..60}, 256^2 detector.  Two forms of one data-term evaluation:
-    the direct and transpose grid kernels (tiles autotuned) captured in a
-    CUDA graph, and the persistent launch resid = H x - y, grad = H^T resid
-    (trtt_b200_plan3d_wls_grad, tile shape autotuned), which also computes
-    the residual and the FP64 cost."""
+    the direct and transpose kernels (tiles autotuned) captured in a CUDA
+    graph, and the call resid = H x - y, grad = H^T resid
+    (trtt_b200_plan3d_wls_grad, three launches or the persistent one,
+    autotuned), which also computes the residual and the FP64 cost."""
     torch = _torch()
     from . import geometry as G, phantoms as P
     from .projectors import Projector3D
@@ -216,7 +216,7 @@ def gates4d(nt=10, seed=0, replays=5):
         torch.cuda.synchronize()
         best = min(best, a.elapsed_time(b))
     pr.status()
-    # persistent launch on measurements of the projections' size
+    # the data-term call on measurements of the projections' size
     meas = (y * 0.9).contiguous()
     wtimes, wchoice = pr.autotune_wls(xc, meas, reps=2)
     grad = torch.zeros_like(xc)
@@ -238,8 +238,8 @@ def gates4d(nt=10, seed=0, replays=5):
                            "autotune_ms": {str(k): v for k, v in wtimes.items()},
                            "ms": wbest, "projections_per_s": 2 * nviews / (wbest / 1e3),
                            "cost": float(cost.item()),
-                           "what": "resid = H x - y, 1/2 |resid|^2 (FP64), grad = H^T resid, "
-                                   "one cooperative launch"}}
+                           "what": "resid = H x - y, 1/2 |resid|^2 (FP64), grad = H^T resid in one call; "
+                                   "(0, 0): three launches, else the persistent launch of that shape"}}
 
 
 def _log(msg):
