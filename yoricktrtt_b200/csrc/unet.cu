@@ -1208,6 +1208,7 @@ struct WgradRowArgs {
   long blocks;          // KT-row stages in all
   int kt, steps;        // rows per stage, stages per CTA
   int a_bytes, stage_bytes, nstg;
+  int accs;             // accumulators that the stages take in turn, 1 or 2
   uint32_t tmem_cols;
 };
 struct WgradRowMaps {
@@ -1297,12 +1298,12 @@ __global__ void __launch_bounds__(128) k_conv3_wgrad_rows(const WgradRowArgs a, 
           const uint64_t ad = tc::sdesc_swz_mn(as + 2u * set * ra, ra, ra);
           const uint32_t alo = uniform((uint32_t)ad), ahi = uniform((uint32_t)(ad >> 32));
           const uint32_t blo = uniform((uint32_t)bd), bhi = uniform((uint32_t)(bd >> 32));
-          const uint32_t acc = uniform(tmem + (uint32_t)(3 * (set * a.cin + ch)));
+          const uint32_t acc = uniform(tmem + (uint32_t)(3 * (((it & (a.accs - 1)) * a.sets + set) * a.cin + ch)));
           // 16 rows per MMA; descriptors count 16 bytes
 #pragma unroll 8
           for (int ks = 0; ks < KT / 16; ++ks)
             tc::mma_bf16_warp(acc, alo + (uint32_t)ks * ra, ahi, blo + (uint32_t)ks * rb, bhi, idesc,
-                              (it > 0 || ks > 0) ? 1u : 0u);
+                              (it >= a.accs || ks > 0) ? 1u : 0u);
         }
         bs += ((uint32_t)(KT + 2 * wp) * rb + 1023u) & ~1023u;
         ch += ic;
@@ -1329,7 +1330,14 @@ __global__ void __launch_bounds__(128) k_conv3_wgrad_rows(const WgradRowArgs a, 
         for (int dy = 0; dy < 3; ++dy)
           for (int j = 0; j < ic; j += 16) {
             float v[16];
-            tc::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(3 * (set * a.cin + ch) + dy * ic + j), v);
+            const uint32_t at = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(3 * (set * a.cin + ch) + dy * ic + j);
+            tc::tmem_ld16(at, v);
+            if (a.accs > 1 && T > 1) {
+              float u[16];
+              tc::tmem_ld16(at + (uint32_t)(3 * a.sets * a.cin), u);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) v[i] += u[i];
+            }
             if (s <= 2) {
               float4 *o = reinterpret_cast<float4 *>(dst + (long)dy * 3 * a.cin + ch + j);
 #pragma unroll
@@ -1867,11 +1875,20 @@ WgradPlan wgrad_plan(int cout, int cin, const Grid3 &g, bool tma = false)
 
 // Layout of k_conv3_wgrad_rows; false where it does not apply.  256 rows per stage
 // where three stages leave room for two CTAs on an SM, else 128 (the X slab's 2 wp
-// extra rows weigh more, but two CTAs overlap their waits); one wave of CTAs.  Below
+// extra rows weigh more, but two CTAs overlap their waits).  Below
 // 4096 rows the 9 per-tap CTAs of a range are faster than 3 (64 -> 64 at 8^3 25.6
 // us against 29.7; at 16^3 all are faster here).
+// Sums in tensor memory round toward zero at every MMA, so the rows that one
+// accumulator takes set the error.  They are at most those of the per-tap kernel's
+// plan: two accumulators in turn where the columns allow it, else more waves of
+// CTAs.  Relative error against float64 with one wave of one accumulator -> now
+// (per-tap kernel): 16 -> 16 at 128^3 2.5e-5 -> 6.0e-6 (1.2e-5), 32 -> 32 at 2 x
+// 64^3 6.1e-6 -> 2.9e-6 (4.4e-6), 64 -> 64 at 64^3 6.0e-6 -> 1.9e-6 (2.1e-6).  The
+// second accumulator costs nothing (106 -> 111 and 58 -> 58 us), the waves, at 64
+// outputs or 96 inputs, 10 to 40% (64 -> 64 at 32^3 36 -> 47, at 64^3 78 -> 111 us;
+// per tap 57 and 226).
 struct WgradRowPlan {
-  int kt, a_bytes, stage_bytes, nstg, smem, sets;
+  int kt, a_bytes, stage_bytes, nstg, smem, sets, accs;
   long chunks, steps, blocks;
   uint32_t tmem_cols;
 };
@@ -1880,8 +1897,11 @@ bool wgrad_row_plan(int cout, int c1, int c2, const Grid3 &g, WgradRowPlan &p)
   const int cin = c1 + c2;
   if (cout != 16 && cout != 32 && cout != 64) return false;
   p.sets = cout == 64 ? 2 : 1;
-  if (p.sets * 3 * cin > 512 || g.wp >= 2048 || g.rows < 4096 || g.rows + 4096 + g.plane >= 0x7FFFFFFFL) return false;
-  p.tmem_cols = pow2_cols(p.sets * 3 * cin);
+  const int cols = p.sets * 3 * cin;
+  if (cols > 512 || g.wp >= 2048 || g.rows < 4096 || g.rows + 4096 + g.plane >= 0x7FFFFFFFL) return false;
+  const bool pair = cols <= 256;
+  p.accs = 2 * cols <= (pair ? 256 : 512) ? 2 : 1;
+  p.tmem_cols = pow2_cols(p.accs * cols);
   auto layout = [&](int kt) {
     auto up = [](int b) { return (b + 1023) & ~1023; };
     p.kt = kt;
@@ -1893,18 +1913,20 @@ bool wgrad_row_plan(int cout, int c1, int c2, const Grid3 &g, WgradRowPlan &p)
       ch += ic;
     }
   };
-  const bool pair = p.tmem_cols <= 256;
+  const WgradPlan tap = wgrad_plan(cout, cin, g, true);
+  const long most_rows = tap.steps * tap.kt;  // per accumulator
   const int half = 110 * 1024, whole = 224 * 1024;
   layout(256);
-  if (!(pair && 3 * p.stage_bytes <= half)) layout(128);
+  if (!(pair && 3 * p.stage_bytes <= half) || most_rows < 256) layout(128);
   const int room = pair && 2 * p.stage_bytes <= half ? half : whole;
   p.nstg = std::min(4, room / p.stage_bytes);
   if (p.nstg < 2) return false;
   p.smem = residency_smem(p.nstg * p.stage_bytes, p.tmem_cols);
   if (p.smem > 226 * 1024) return false;
   p.blocks = (g.rows - 2 * g.plane + p.kt - 1) / p.kt;
-  const long ctas = 148L * (2 * (p.smem + 2048) <= 227 * 1024 && pair ? 2 : 1);
-  const long most = std::min(p.blocks, std::max(1L, ctas / 3));
+  const long wave = 148L * (2 * (p.smem + 2048) <= 227 * 1024 && pair ? 2 : 1) / 3;
+  const long need = (p.blocks + p.accs * (most_rows / p.kt) - 1) / (p.accs * (most_rows / p.kt));
+  const long most = std::min(p.blocks, (need + wave - 1) / wave * wave);
   p.steps = (p.blocks + most - 1) / most;
   p.chunks = (p.blocks + p.steps - 1) / p.steps;
   return true;
@@ -2079,11 +2101,12 @@ int trtt_b200_conv3_plan_info(int which, int cin, int cout, int nb, int d, int h
 size_t trtt_b200_conv3_wgrad_scratch(int cout, int cin, int nb, int d, int h, int w)
 {
   if (!grid_ok(nb, d, h, w) || cout <= 0 || cin <= 0 || cout % 8 || cin % 8) return 0;
-  // enough for every kernel
+  // enough for every kernel and every split of the input channels over two tensors
   const Grid3 g = make_grid(nb, d, h, w);
   long chunks = std::max(wgrad_plan(cout, cin, g, false).chunks, wgrad_plan(cout, cin, g, true).chunks);
-  // (k_conv3_wgrad_rows: at most two CTAs per SM over three dz)
-  chunks = std::max(chunks, std::min((g.rows - 2 * g.plane + 127) / 128, 2L * 148 / 3));
+  WgradRowPlan rp;
+  for (int c1 = 16; c1 <= cin && cin % 16 == 0; c1 += 16)
+    if (wgrad_row_plan(cout, c1, cin - c1, g, rp)) chunks = std::max(chunks, rp.chunks);
   return (size_t)chunks * cout * 27 * cin * sizeof(float);
 }
 
@@ -2131,6 +2154,7 @@ int trtt_b200_conv3_wgrad(const void *dy, int cout, const void *x1, int c1, cons
     r.a_bytes = rp.a_bytes;
     r.stage_bytes = rp.stage_bytes;
     r.nstg = rp.nstg;
+    r.accs = rp.accs;
     r.tmem_cols = rp.tmem_cols;
     WgradRowMaps maps;
     std::memset(&maps, 0, sizeof(maps));
