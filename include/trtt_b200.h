@@ -534,7 +534,14 @@ int trtt_b200_cb3d_cubic_forward_noalloc(const float *vol_columns, float *sino,
  * unet_status: -1 if a convolution kernel gave up waiting for its tensor-core
  *   work (bounded waits), then clears the flag; synchronises the stream. */
 int trtt_b200_conv3_pack(const float *w, int cout, int cin, int transpose, void *wpack, void *stream);
-/* Staging of trtt_b200_conv3_forward, process-wide: 0 copies each stage's
+/* Kernels of the convolutions, process-wide.  Default (on < 0): the forward
+ * kernel streamed along z (16 outputs; 32 with two stages a plane or more and
+ * rows of at most 148 voxels) and the weight gradient with fused rows (16, 32 or
+ * 64 outputs, 4096 padded rows or more); shapes that they do not take run as with
+ * on = 2, or 0 where the driver provides no tensor-map encoder.  They fuse taps
+ * into one MMA and sum in another order than the others: results differ in
+ * rounding.  on >= 0 selects a staging of the per-tap kernels instead, which
+ * compute the same MMAs in the same order as one another: 0 copies each stage's
  * slab and weights into shared memory with 16-byte cp.async by all 128
  * threads; 1 loads them with TMA (2D tiled copies of the padded
  * channels-last activations, a bulk copy of the weights) issued by one
@@ -542,14 +549,12 @@ int trtt_b200_conv3_pack(const float *w, int cout, int cin, int transpose, void 
  * (warp specialisation), one tile per CTA; 2 is the same in persistent
  * CTAs of 6 warps that walk many tiles with two tensor-memory accumulators,
  * the epilogue of one tile (4 warps) overlapping the copies and MMAs of the
- * next (needs 2 x 2 x n <= 512 tensor-memory columns; else 1).  All
- * compute the same MMAs in the same order (identical results).  Forward
- * pass of the 128^3 U-Net: 1.73 ms (0), 1.37 ms (1), 1.03 ms (2).  The
- * weight gradient follows the same switch: 0 stages with cp.async, any
- * other value with TMA and a producer / MMA-issuer pair (same MMAs; a
- * training step of the 128^3 U-Net 8.6 ms with 0, 5.4 ms with TMA).
- * Default (on < 0): 2 when the driver provides a tensor-map encoder, else
- * 0.  -1 when asked for TMA without one.  No counterpart in the reference. */
+ * next (needs 2 x 2 x n <= 512 tensor-memory columns; else 1).  The weight
+ * gradient follows the same switch: 0 stages with cp.async, 1 and 2 with TMA
+ * and a producer / MMA-issuer pair.  128^3 U-Net: forward pass 1.73 ms (0),
+ * 1.37 ms (1), 1.03 ms (2), 0.71 ms (default); training step 8.6 ms (0), 5.4 ms
+ * (2), 2.6 ms (default).  -1 when asked for TMA without an encoder.  No
+ * counterpart in the reference. */
 int trtt_b200_conv3_set_tma(int on);
 int trtt_b200_conv3_forward(const void *x1, int c1, const void *x2, int c2, const void *wpack, int n,
                             const float *bias, int mode, float slope, void *y, void *y2, int n1,
@@ -565,7 +570,14 @@ size_t trtt_b200_conv3_wgrad_scratch(int cout, int cin, int nb, int d, int h, in
  * stages, dynamic shared memory, tensor-memory columns, row chunks, stages
  * per chunk.  which = 0 and 1 describe the cp.async staging; which = 2 the
  * persistent TMA forward kernel (layout of 0), which = 3 the TMA weight
- * gradient (layout of 1). */
+ * gradient (layout of 1).  which = 4: forward kernel streamed along z,
+ * info[0..9] = sub-tiles S, slab rows, stage bytes, stages, bytes of weights and
+ * of edge rows ahead of them, dynamic shared memory, tensor-memory columns,
+ * tiles per plane, planes per z segment.  which = 5: weight gradient with fused
+ * rows, info[0..9] = rows per stage, A bytes and bytes of a stage, stages,
+ * dynamic shared memory, tensor-memory columns, MMAs along M, accumulators, row
+ * chunks, stages per chunk.  -1 where those two do not take the shape (4 and 5
+ * take all input channels as one tensor). */
 int trtt_b200_conv3_plan_info(int which, int cin, int cout, int nb, int d, int h, int w, long *info);
 int trtt_b200_conv3_wgrad(const void *dy, int cout, const void *x1, int c1, const void *x2, int c2,
                           float *dw, float *db, void *scratch, size_t scratch_bytes, int nb, int d,

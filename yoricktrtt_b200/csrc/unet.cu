@@ -2094,8 +2094,23 @@ int trtt_b200_conv3_plan_info(int which, int cin, int cout, int nb, int d, int h
     for (int i = 0; i < 8; ++i) info[i] = v[i];
     return 0;
   }
-  return fail("conv3_plan_info: which must be 0 (forward, cp.async), 1 (weight gradient, cp.async), "
-              "2 (forward, persistent TMA) or 3 (weight gradient, TMA)");
+  if (which == 4) {
+    FwdPlan p;
+    ZArgs z;
+    if (!fwd_plan_z(cout, cin, 0, g, p, z)) return fail("conv3_plan_info: the z-streaming kernel does not take this shape");
+    const long v[] = {z.S, p.rh, p.stage_bytes, p.nstg, z.w_bytes, z.edge_bytes, p.smem, p.tmem_cols, z.tiles, z.len};
+    for (int i = 0; i < 10; ++i) info[i] = v[i];
+    return 0;
+  }
+  if (which == 5) {
+    WgradRowPlan p;
+    if (!wgrad_row_plan(cout, cin, 0, g, p)) return fail("conv3_plan_info: the row-fused kernel does not take this shape");
+    const long v[] = {p.kt, p.a_bytes, p.stage_bytes, p.nstg, p.smem, p.tmem_cols, p.sets, p.accs, p.chunks, p.steps};
+    for (int i = 0; i < 10; ++i) info[i] = v[i];
+    return 0;
+  }
+  return fail("conv3_plan_info: which must be 0 (forward, cp.async), 1 (weight gradient, cp.async), 2 (forward, "
+              "persistent TMA), 3 (weight gradient, TMA), 4 (forward, streamed along z) or 5 (weight gradient, rows)");
 }
 
 size_t trtt_b200_conv3_wgrad_scratch(int cout, int cin, int nb, int d, int h, int w)
