@@ -374,8 +374,11 @@ __global__ void __launch_bounds__(32 * kWarps, 3) k_fwd2d_orbit(const Orbit2DLau
           if (distinct) {
             for (int l = 0; l < Lw; ++l) {
               const int c = ft.f + l;
-              const float w = (float)(wk.weight(A, ft, c) * ft.amp);
-              if (l < L && c >= u0) {
+              const double wd = wk.weight(A, ft, c);
+              const float w = (float)(wd * ft.amp);
+              // (the ends of a Long-Fessler range may have weight 0: no cells of the
+              // footprint, for values that are not finite)
+              if (l < L && c >= u0 && (MODEL != M2_LF || wd != 0.0)) {
                 V v = row[c - u0];
                 vfma(v, w, x);
                 row[c - u0] = v;
@@ -385,8 +388,9 @@ __global__ void __launch_bounds__(32 * kWarps, 3) k_fwd2d_orbit(const Orbit2DLau
           } else {
             for (int l = 0; l < L; ++l) {
               const int c = ft.f + l;
-              const float w = (float)(wk.weight(A, ft, c) * ft.amp);
-              if (c >= u0) {
+              const double wd = wk.weight(A, ft, c);
+              const float w = (float)(wd * ft.amp);
+              if (c >= u0 && (MODEL != M2_LF || wd != 0.0)) {
 #pragma unroll
                 for (int s = 0; s < NS; ++s)
                   atomicAdd(reinterpret_cast<float *>(row + (c - u0)) + s, w * x[s]);
