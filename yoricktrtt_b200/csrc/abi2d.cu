@@ -777,7 +777,8 @@ extern "C" int trtt_b200_plan2d_forward(trtt_b200_plan2d *pl, const float *img, 
   if (!pl || !img || !sino) return fail("plan2d_forward: null argument");
   cudaStream_t st = (cudaStream_t)stream;
   if (!pl->orbit.groups.empty())
-    TRTT_CK(launch_fwd2d_orbit(orbit_launch(pl->orbit, pl->groups.as<Orbit2D>(), pl->P, pl->views.as<View2D>(), img, sino), st));
+    TRTT_CK(launch_fwd2d_orbit(
+        orbit_launch(pl->orbit, pl->groups.as<Orbit2D>(), pl->P, pl->views.as<View2D>(), img, sino), st));
   else if (pl->lf)
     TRTT_CK(launch_lf_fwd(pl->views.as<LFView>(), (int)pl->nviews, (int)pl->ndet, pl->line, img, sino, st));
   else
@@ -793,7 +794,8 @@ extern "C" int trtt_b200_plan2d_backward(trtt_b200_plan2d *pl, const float *sino
   if (!pl || !img || !sino) return fail("plan2d_backward: null argument");
   cudaStream_t st = (cudaStream_t)stream;
   if (!pl->orbit.groups.empty())
-    TRTT_CK(launch_back2d_orbit(orbit_launch(pl->orbit, pl->groups.as<Orbit2D>(), pl->P, pl->views.as<View2D>(), sino, img), st));
+    TRTT_CK(launch_back2d_orbit(
+        orbit_launch(pl->orbit, pl->groups.as<Orbit2D>(), pl->P, pl->views.as<View2D>(), sino, img), st));
   else if (pl->lf)
     TRTT_CK(launch_lf_back(pl->views.as<LFView>(), (int)pl->nviews, (int)pl->npix, pl->line, sino, img, st));
   else

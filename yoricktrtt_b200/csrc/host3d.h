@@ -289,7 +289,8 @@ inline SweepBounds sweep_bounds(const Params3D &P, const View3D *views, long nvi
   if (P.model == MODEL_TABLE && !(hmin > 0.0 && (2.0 * hsu + 20.0 + std::fabs(P.coord0)) / (hmin * P.step) < 1e9 &&
                                   (2.0 * P.hs0 + std::fabs(P.coord0)) / P.step < 1e9))
     return b;
-  if (!(hsv > 0.0 && hsv < 1e4 && hsu < 1e4 && b.du < 1e6 && b.dcol < 1e6 && u0 > -1e8 && u1 < 1e8 && v0 > -1e8 && v1 < 1e8)) return b;
+  if (!(hsv > 0.0 && hsv < 1e4 && hsu < 1e4 && b.du < 1e6 && b.dcol < 1e6)) return b;
+  if (!(u0 > -1e8 && u1 < 1e8 && v0 > -1e8 && v1 < 1e8)) return b;
   b.rows = (int)std::floor(2.0 * hsv * 1.0001) + 2;
   b.u0 = (int)std::fmin(std::fmax(std::floor(u0 - hsu * 1.0001) - 1.0, 0.0), P.nu);
   b.u1 = (int)std::fmin(std::fmax(std::ceil(u1 + hsu * 1.0001) + 2.0, 0.0), P.nu);

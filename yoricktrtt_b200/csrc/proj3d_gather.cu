@@ -66,8 +66,8 @@ template <> struct GatherRec<MODEL_TABLE> {
 };
 template <int MODEL> __host__ __device__ constexpr size_t gather_warp_bytes(int cap)
 {
-  return GatherRec<MODEL>::batch * kNC * sizeof(typename GatherRec<MODEL>::T) + sizeof(float2) * kTabRows * kNC + sizeof(float) * kNC * gather_row(cap) +
-         32;
+  return GatherRec<MODEL>::batch * kNC * sizeof(typename GatherRec<MODEL>::T) + sizeof(float2) * kTabRows * kNC +
+         sizeof(float) * kNC * gather_row(cap) + 32;
 }
 
 template <int GEOM>
@@ -321,7 +321,8 @@ k_back3d_gather(const __grid_constant__ GatherLaunch A)
       const bool on = r.view >= 0;
       const int view = __reduce_max_sync(FULLM, r.view);
       if (view < 0) continue;
-      const int r0 = __reduce_min_sync(FULLM, on ? r.lo : INT_MAX), r1 = __reduce_max_sync(FULLM, on ? r.lo + r.n : INT_MIN);
+      const int r0 = __reduce_min_sync(FULLM, on ? r.lo : INT_MAX);
+      const int r1 = __reduce_max_sync(FULLM, on ? r.lo + r.n : INT_MIN);
       int c0 = __reduce_min_sync(FULLM, r.c0) & ~3, c1 = __reduce_max_sync(FULLM, r.c1);
       if (A.vec4) c1 = (c1 + 3) & ~3;
       if (c1 - c0 > A.cap) {  // more cells than the launcher's bound: never in a correct run
@@ -665,7 +666,8 @@ cudaError_t launch(GatherLaunch L, cudaStream_t st)
   // their half supports
   const double len = L.b.du * 2 * kH * PP + L.b.dcol * (kNC - 1) + 2.0 * L.b.hsu + 16.0;
   L.cap = len < (double)L.P.nu ? (int)len : (L.P.nu + 3) & ~3;
-  const size_t smem = table_bytes(L.P) + std::max(kWarps * gather_warp_bytes<MODEL>(L.cap), sizeof(float2) * 2 * PP * 32 * kWarps);
+  const size_t smem = table_bytes(L.P) +
+                      std::max(kWarps * gather_warp_bytes<MODEL>(L.cap), sizeof(float2) * 2 * PP * 32 * kWarps);
   if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
   const dim3 grid((unsigned)((groups * L.vsplit + kWarps - 1) / kWarps), (unsigned)chunks);
   auto go = [&](auto kern) {
@@ -715,8 +717,10 @@ bool gather_fits(const Params3D &P, const SweepBounds &b)
   if (P.model == MODEL_TABLE)
     return b.rows > 0 && table_slots(P) <= kTableSlots && (P.nz + 1) / 2 / kH < 65535 &&
            table_bytes(P) + GatherRec<MODEL_TABLE>::warps * gather_warp_bytes<MODEL_TABLE>(cap) <= 227 * 1024;
-  return b.rows > 0 && GatherRec<MODEL_CUBIC>::warps * gather_warp_bytes<MODEL_CUBIC>(cap) <= 113 * 1024 && (P.nz + 1) / 2 / kH < 65535 &&
-         2.0 * b.hsu + b.du + 4.0 < 2.0 * kSweepGuard - 16.0;
+  // (the last test: a walk over two voxels' cells fits the zeros beside a profile,
+  // voxels of up to about 2.4 cells on the detector)
+  return b.rows > 0 && GatherRec<MODEL_CUBIC>::warps * gather_warp_bytes<MODEL_CUBIC>(cap) <= 113 * 1024 &&
+         (P.nz + 1) / 2 / kH < 65535 && 2.0 * b.hsu + b.du + 4.0 < 2.0 * kSweepGuard - 16.0;
 }
 
 cudaError_t launch_back3d_gather(const GatherLaunch &L, cudaStream_t st)

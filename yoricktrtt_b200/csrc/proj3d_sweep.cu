@@ -1,6 +1,7 @@
-// proj3d_sweep.cu -- direct 3D projection of column-factorised views: launches of the sweep item (sweep3d.cuh) over (view or
-// view group, band of detector rows, u tile), the image lines of a tile shared
-// by a cluster of CTAs where there are too few tiles for the SMs.
+// proj3d_sweep.cu -- direct 3D projection of column-factorised views: launches
+// of the sweep item (sweep3d.cuh) over (view or view group, band of detector
+// rows, u tile), the image lines of a tile shared by a cluster of CTAs where
+// there are too few tiles for the SMs.
 //
 // Measured (B200; the band kernel of proj3d_fast.cu, for groups the kernel of
 // proj3d_group.cu before):

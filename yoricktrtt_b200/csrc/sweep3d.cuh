@@ -1,9 +1,9 @@
 // sweep3d.cuh -- direct projection of column-factorised views (closed-form
-// footprint; tabulated footprint with the walks of table3d.cuh): the band of detector cells [v0, v1) x [u0, u1) of G views related by
-// turns of the grid (find_view_groups, host3d.h; G = 1: one view), accumulated
-// in shared memory, the members' values of a cell side by side.  The footprints
-// are those of the first view; member m sees there the columns turned back by
-// its turn.
+// footprint; tabulated footprint with the walks of table3d.cuh): the band of
+// detector cells [v0, v1) x [u0, u1) of G views related by turns of the grid
+// (find_view_groups, host3d.h; G = 1: one view), accumulated in shared memory,
+// the members' values of a cell side by side.  The footprints are those of the
+// first view; member m sees there the columns turned back by its turn.
 //
 // A warp sweeps an image line of voxel columns (along i or j, the axis on which
 // neighbouring columns project further apart), NC = 32 / H consecutive columns
@@ -150,8 +150,8 @@ template <int Q, int H> struct SweepStrip {
 };
 
 // Shared memory of one CTA: the band (rows rounded up to whole lock groups),
-// one lock per group and strip, and per warp the records of a batch of columns, a table
-// of row weights and NC profile rows with guards around them.
+// one lock per group and strip, and per warp the records of a batch of columns, a
+// table of row weights and NC profile rows with guards around them.
 template <int MODEL> struct SweepRec {
   using T = SweepCol;
   static constexpr int batch = 32;  // columns whose records are built together
@@ -275,8 +275,9 @@ __device__ __forceinline__ bool sweep_record(const Params3D &P, const View3D &V,
 __device__ __forceinline__ bool is_finite(float x) { return fabsf(x) < __int_as_float(0x7f800000); }
 
 // A lane's walk: `steps` double cells from cell `rel` of the row, voxels a and
-// c with abscissae ax and cx at the second edge and steps da, dc per cell.  CHECK: cells outside [0, ncell) are left alone (some
-// lane's walk leaves the row's guards).  All lanes of the warp take it.
+// c with abscissae ax and cx at the second edge and steps da, dc per cell.  CHECK:
+// cells outside [0, ncell) are left alone (some lane's walk leaves the row's
+// guards).  All lanes of the warp take it.
 template <int G, bool CHECK>
 __device__ __forceinline__ void sweep_walk(typename SweepVec<G>::T *row, int rel, int ncell, int steps, float ax,
                                            float cx, float da, float dc, const float (&xa)[G], const float (&xc)[G])
@@ -367,8 +368,9 @@ __device__ __forceinline__ float gate_value(const View3D &V, const float *colp, 
 
 // Profiles of a warp's columns, tabulated footprint: H lanes per column, each
 // one voxel per pass, neighbouring lanes at least two cells apart, so that a
-// step of two cells writes distinct cells.  row: the column's profile row; returns the lanes that
-// had voxels to add.
+// step of two cells writes distinct cells.  row: the column's profile row; *odd is
+// set where a voxel is not finite (left out).  Returns the lanes that had voxels to
+// add.
 template <int GEOM, int H>
 __device__ __forceinline__ unsigned table_profiles(const Params3D &P, const View3D &V, const TableSh &T,
                                                    const TableCol &r, bool mine, int q, const float *colp, long dgate,
@@ -779,8 +781,9 @@ __device__ __noinline__ void sweep_odd(const Params3D &P, const View3D &V, const
                 w = (float)(table_at(T, dadd(t.start, dmul(e + 1.0, t.inc))) -
                             table_at(T, dadd(t.start, dmul(e, t.inc))));
               } else {
-                const float a = l == 0 ? first_edge_prim2(up).x : cubic_prim2(f2(fmaf((float)l, up.inc.x, up.start.x))).x;
-                w = cubic_prim2(f2(fmaf((float)(l + 1), up.inc.x, up.start.x))).x - a;
+                const float2 e = fma2(make_float2((float)l, (float)(l + 1)), f2(up.inc.x), f2(up.start.x));
+                const float2 F = cubic_prim2(e);
+                w = F.y - (l == 0 ? first_edge_prim2(up).x : F.x);
               }
               float xm = 0.f;
               for (int m = 0; m < G; ++m)

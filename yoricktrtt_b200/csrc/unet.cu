@@ -121,55 +121,55 @@ struct FwdArgs {
 __device__ __forceinline__ void fwd_emit(const FwdArgs &a, long p, int j, float (&v)[16])
 {
   const int n = a.n;
-        if (a.bias && a.mode != kFwdGrad) {
-  #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] += a.bias[j + i];
-        }
-        if (a.mode == kFwdAct) {
-          uint4 q0, q1;
-          q0.x = pack_bf16x2(act(v[0], a.slope), act(v[1], a.slope));
-          q0.y = pack_bf16x2(act(v[2], a.slope), act(v[3], a.slope));
-          q0.z = pack_bf16x2(act(v[4], a.slope), act(v[5], a.slope));
-          q0.w = pack_bf16x2(act(v[6], a.slope), act(v[7], a.slope));
-          q1.x = pack_bf16x2(act(v[8], a.slope), act(v[9], a.slope));
-          q1.y = pack_bf16x2(act(v[10], a.slope), act(v[11], a.slope));
-          q1.z = pack_bf16x2(act(v[12], a.slope), act(v[13], a.slope));
-          q1.w = pack_bf16x2(act(v[14], a.slope), act(v[15], a.slope));
-          uint4 *dst = reinterpret_cast<uint4 *>(static_cast<bf16 *>(a.y) + p * n + j);
-          dst[0] = q0;
-          dst[1] = q1;
-        } else if (a.mode == kFwdF32) {
-          float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(a.y) + p * n + j);
-  #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            dst[i] = make_float4(act(v[4 * i], a.slope), act(v[4 * i + 1], a.slope),
-                                 act(v[4 * i + 2], a.slope), act(v[4 * i + 3], a.slope));
-        } else if (a.mode == kFwdHead) {
-          if (j == 0) static_cast<float *>(a.y)[p] = a.resid[p] + v[0];
-        } else {  // kFwdGrad
-          bf16 *base;
-          int ld, c0;
-          if (j < a.n1) { base = static_cast<bf16 *>(a.y); ld = a.n1; c0 = j; }
-          else { base = static_cast<bf16 *>(a.y2); ld = n - a.n1; c0 = j - a.n1; }
-          uint4 *dst = reinterpret_cast<uint4 *>(base + p * ld + c0);
-          if (a.accumulate) {
-            const uint4 o0 = dst[0], o1 = dst[1];
-            const uint32_t ow[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
-  #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const float2 f = unpack_bf16x2(ow[i]);
-              v[2 * i] += f.x;
-              v[2 * i + 1] += f.y;
-            }
-          }
-          uint4 q0, q1;
-          q0.x = pack_bf16x2(v[0], v[1]); q0.y = pack_bf16x2(v[2], v[3]);
-          q0.z = pack_bf16x2(v[4], v[5]); q0.w = pack_bf16x2(v[6], v[7]);
-          q1.x = pack_bf16x2(v[8], v[9]); q1.y = pack_bf16x2(v[10], v[11]);
-          q1.z = pack_bf16x2(v[12], v[13]); q1.w = pack_bf16x2(v[14], v[15]);
-          dst[0] = q0;
-          dst[1] = q1;
-        }
+  if (a.bias && a.mode != kFwdGrad) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] += a.bias[j + i];
+  }
+  if (a.mode == kFwdAct) {
+    uint4 q0, q1;
+    q0.x = pack_bf16x2(act(v[0], a.slope), act(v[1], a.slope));
+    q0.y = pack_bf16x2(act(v[2], a.slope), act(v[3], a.slope));
+    q0.z = pack_bf16x2(act(v[4], a.slope), act(v[5], a.slope));
+    q0.w = pack_bf16x2(act(v[6], a.slope), act(v[7], a.slope));
+    q1.x = pack_bf16x2(act(v[8], a.slope), act(v[9], a.slope));
+    q1.y = pack_bf16x2(act(v[10], a.slope), act(v[11], a.slope));
+    q1.z = pack_bf16x2(act(v[12], a.slope), act(v[13], a.slope));
+    q1.w = pack_bf16x2(act(v[14], a.slope), act(v[15], a.slope));
+    uint4 *dst = reinterpret_cast<uint4 *>(static_cast<bf16 *>(a.y) + p * n + j);
+    dst[0] = q0;
+    dst[1] = q1;
+  } else if (a.mode == kFwdF32) {
+    float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(a.y) + p * n + j);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      dst[i] = make_float4(act(v[4 * i], a.slope), act(v[4 * i + 1], a.slope),
+                           act(v[4 * i + 2], a.slope), act(v[4 * i + 3], a.slope));
+  } else if (a.mode == kFwdHead) {
+    if (j == 0) static_cast<float *>(a.y)[p] = a.resid[p] + v[0];
+  } else {  // kFwdGrad
+    bf16 *base;
+    int ld, c0;
+    if (j < a.n1) { base = static_cast<bf16 *>(a.y); ld = a.n1; c0 = j; }
+    else { base = static_cast<bf16 *>(a.y2); ld = n - a.n1; c0 = j - a.n1; }
+    uint4 *dst = reinterpret_cast<uint4 *>(base + p * ld + c0);
+    if (a.accumulate) {
+      const uint4 o0 = dst[0], o1 = dst[1];
+      const uint32_t ow[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 f = unpack_bf16x2(ow[i]);
+        v[2 * i] += f.x;
+        v[2 * i + 1] += f.y;
+      }
+    }
+    uint4 q0, q1;
+    q0.x = pack_bf16x2(v[0], v[1]); q0.y = pack_bf16x2(v[2], v[3]);
+    q0.z = pack_bf16x2(v[4], v[5]); q0.w = pack_bf16x2(v[6], v[7]);
+    q1.x = pack_bf16x2(v[8], v[9]); q1.y = pack_bf16x2(v[10], v[11]);
+    q1.z = pack_bf16x2(v[12], v[13]); q1.w = pack_bf16x2(v[14], v[15]);
+    dst[0] = q0;
+    dst[1] = q1;
+  }
 }
 
 // Epilogue of the forward / input-gradient convolution: the S accumulators
@@ -595,9 +595,8 @@ __global__ void __launch_bounds__(192) k_conv3_fwd_pers(const FwdArgs a, const _
 // shuffles, and the rows at a warp's edge through shared memory): 9 MMAs per 16
 // channels and 128 rows, not 27.  All weights stay in shared memory.
 //   4 S HW warps (S = 1: two such sets, by turns): epilogue, warp (s, q, j): 32
-//     rows 128 s + 32 q, channels
-//     [j, j + 16): it takes its three blocks to registers, which frees the
-//     buffer, and then exchanges rows and writes;
+//     rows from 128 s + 32 q, channels [j, j + 16): it takes its three blocks to
+//     registers, which frees the buffer, and then exchanges rows and writes;
 //   warp EW, one thread: producer, stages (input plane, 16 to 64 channels) into
 //     the ring by TMA, a row's channels as 32, 64 or 128 bytes in the swizzle of
 //     that width.  Boxes of 8 channels would write 16 bytes of shared memory per
@@ -647,9 +646,11 @@ struct RingPos {
 };
 
 template <int S, int HW, int NB>
-__global__ void __launch_bounds__(z_threads(S, HW), 1) k_conv3_fwd_z(const FwdArgs a, const ZArgs z, const __grid_constant__ FwdMaps maps)
+__global__ void __launch_bounds__(z_threads(S, HW), 1)
+k_conv3_fwd_z(const FwdArgs a, const ZArgs z, const __grid_constant__ FwdMaps maps)
 {
-  constexpr int ES = z_sets(S), EP = 4 * S * HW, EW = EP * ES;  // epilogue warps (EP a set); then the producer and the issuers
+  // epilogue warps (EP a set); then the producer and the issuers
+  constexpr int ES = z_sets(S), EP = 4 * S * HW, EW = EP * ES;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t full[kZStages], empty[kZStages], accf[NB], acce[NB], edgeb[ES], finb;
   __shared__ uint32_t s_taddr;
@@ -1267,7 +1268,8 @@ __global__ void __launch_bounds__(128) k_conv3_wgrad_rows(const WgradRowArgs a, 
           const uint32_t rb = 2u * ic;
           for (int r = 0; r < rows; r += 128)
             tc::tma_load_2d(dst + (uint32_t)r * rb,
-                            first ? (rows - r >= 128 ? &maps.x1 : &maps.x1_tail) : (rows - r >= 128 ? &maps.x2 : &maps.x2_tail),
+                            first ? (rows - r >= 128 ? &maps.x1 : &maps.x1_tail)
+                                  : (rows - r >= 128 ? &maps.x2 : &maps.x2_tail),
                             x, xr + r, &full[p.slot]);
           dst += ((uint32_t)rows * rb + 1023u) & ~1023u;
           ch += ic;
@@ -1342,7 +1344,8 @@ __global__ void __launch_bounds__(128) k_conv3_wgrad_rows(const WgradRowArgs a, 
               float4 *o = reinterpret_cast<float4 *>(dst + (long)dy * 3 * a.cin + ch + j);
 #pragma unroll
               for (int i = 0; i < 4; ++i)
-                o[i] = T > 0 ? make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                o[i] = T > 0 ? make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3])
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
             }
           }
         ch += ic;
@@ -1364,8 +1367,7 @@ __global__ void __launch_bounds__(128) k_conv3_wgrad_rows(const WgradRowArgs a, 
 
 // out[i] = sum over chunks of part[chunk][i]; 32 outputs and 8 threads per output
 // in a block (one thread per output was a chain of ~100 loads: 11.4 -> 4.1 us for 98
-// chunks of 27648).  Clears
-// `zero` (nz floats), which the next kernel adds into.
+// chunks of 27648).  Clears `zero` (nz floats), which the next kernel adds into.
 __global__ void __launch_bounds__(256) k_sum_parts(const float *__restrict__ part, int chunks, long n,
                                                    float *__restrict__ out, float *zero, int nz)
 {
@@ -1738,12 +1740,12 @@ FwdPlan fwd_plan_pers(int n, int groups, const Grid3 &g, int *S)
 }
 
 // Layout of the z-streaming kernel; false where it does not apply: the
-// accumulators in tensor memory, all weights and two stages in shared memory.  Segments of z: fewest waves of CTAs (one per SM) times
-// planes per CTA (two input planes of halo, and about two for start and end).
+// accumulators in tensor memory, all weights and two stages in shared memory.
+// Segments of z: fewest waves of CTAs (one per SM) times planes per CTA (two input
+// planes of halo, and about two for start and end).
 bool fwd_plan_z(int n, int c1, int c2, const Grid3 &g, FwdPlan &p, ZArgs &z)
 {
   const int groups = (c1 + c2) / 16, ic = std::max(z_channels(c1), c2 ? z_channels(c2) : 0);
-
   z.S = n == 16 ? 3 : 1;
   z.hw = n / 16;
   const int nb = n == 32 ? 5 : 3;  // accumulators
