@@ -69,6 +69,14 @@ def test_group_shape_can_be_given_back(ask):
     assert "k_fwd3d_sweep" in _forward(pr)
 
 
+def test_refused_group_tiles_leave_the_default_kernel():
+    from yoricktrtt_b200 import _lib
+    pr = _plan(views=8, theta=False)
+    assert pr.groups() == (0, 0, 2)
+    assert _lib.load().trtt_b200_plan3d_set_group_tiles(pr._h, 8, 0, 0, -1) == -1
+    assert "k_fwd3d_sweep" in _forward(pr)
+
+
 def test_persistent_shape_can_be_given_back():
     import torch
     pr = _plan()

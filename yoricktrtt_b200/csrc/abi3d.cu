@@ -356,12 +356,13 @@ extern "C" int trtt_b200_plan3d_set_group_tiles(trtt_b200_plan3d *pl, int band_r
     if (group_fwd_smem(G, r, utile, group_fwd_warps(G, r, utile, minb)) > 227u * 1024u)
       return fail("plan3d_set_group_tiles: band does not fit in shared memory");
   }
+  if (back_chunk_bytes < 0) return fail("plan3d_set_group_tiles: negative chunk size");
+  // (a request that is refused leaves the plan as it was)
   for (int q = 0; q < 3; ++q)
     if (req[q]) {
       pl->gband[q] = req[q];
       pl->group_set = true;
     }
-  if (back_chunk_bytes < 0) return fail("plan3d_set_group_tiles: negative chunk size");
   if (back_chunk_bytes) pl->back_chunk_bytes = back_chunk_bytes;
   return 0;
 }
