@@ -289,7 +289,7 @@ k_back3d_gather(const __grid_constant__ GatherLaunch A)
     return __any_sync(FULLM, !is_finite(m));
   };
   bool left = false;
-  if (GATED) rest = GatherRest{{0, 0}, {-1, -1}, INT_MAX};
+  if (GATED && lane == 0) rest = GatherRest{{0, 0}, {-1, -1}, INT_MAX};  // (lane 0 alone writes it)
   const int nview = active ? (A.order ? A.norder : A.view_hi - A.view_lo) : 0;
   const int vstep = kBatch * A.vsplit;
   for (int vb = vs * kBatch; vb < nview && !left; vb += vstep) {
@@ -339,7 +339,7 @@ k_back3d_gather(const __grid_constant__ GatherLaunch A)
         if (gp.g0 != ga || (gp.g1 >= 0 && gp.g1 != gb)) {
           if (spoiled()) {
             left = true;
-            rest.next = vb + b;
+            if (lane == 0) rest.next = vb + b;
             break;
           }
           if (gp.g0 == gb) {  // the second gate becomes the first
@@ -358,12 +358,14 @@ k_back3d_gather(const __grid_constant__ GatherLaunch A)
             flush(NA - 1, gb);
           }
           // (slot 1 starts anew in every case; a gate that moves to slot 0 keeps its start)
-          if (gp.g0 != ga) rest.start[0] = gp.g0 == gb ? rest.start[1] : vb + b;
-          rest.start[1] = vb + b;
+          if (lane == 0) {
+            if (gp.g0 != ga) rest.start[0] = gp.g0 == gb ? rest.start[1] : vb + b;
+            rest.start[1] = vb + b;
+            rest.g[0] = gp.g0;
+            rest.g[1] = gp.g1;
+          }
           ga = gp.g0;
           gb = gp.g1;
-          rest.g[0] = ga;
-          rest.g[1] = gb;
         }
       }
       // ---- v-collapsed profiles of the four columns ------------------------
@@ -603,6 +605,7 @@ k_back3d_gather(const __grid_constant__ GatherLaunch A)
     }
   }
   left = left || spoiled();
+  __syncwarp();
   if (GATED) {
     if (!left) {
       flush(0, ga);
