@@ -137,3 +137,42 @@ def test_transpose(oracle_port, case, gates):
             each += b
             hit = np.maximum(hit, h)
     _check(got, each, hit)
+
+
+@pytest.mark.parametrize("mode,views,square,table", [(CONE, 24, False, False), (PAR, 24, False, True),
+                                                     (CONE, 24, True, False), (PAR, 22, True, False)])
+def test_forward_of_nan_volume(oracle_port, mode, views, square, table):
+    """A diverged iterate: every cell that some voxel reaches is NaN, and the call
+    takes the time of a finite volume's up to a factor (16; about 5 expected: a
+    second pass over the columns, with atomics), not that of a pass voxel by voxel
+    (over 100)."""
+    import torch
+    from yoricktrtt_b200.projectors import Projector3D
+    sc, tab = _scan((mode, 64, 64, 60, 120, 96, 1.0, table), views, square=square)
+    pr = Projector3D(sc, tab)
+    vol = torch.rand(pr.volume_shape("columns"), device="cuda")
+    nan = torch.full_like(vol, float("nan"))
+    out = torch.zeros(pr.detector_shape(), device="cuda")
+
+    def ms(x):
+        best = math.inf
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            out.zero_()
+            a.record()
+            pr.forward(x, out=out, layout="columns")
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    base = ms(vol)
+    took = ms(nan)
+    pr.status()
+    got = out.cpu().numpy()
+    for v in (0, views // 3):
+        hit = _oracle(oracle_port, sc, v, np.ones((sc.nz, sc.ny, sc.nx)), 0, tab)
+        odd = np.isnan(got[v])
+        assert not odd[hit == 0.0].any() and odd[hit > 1e-4 * hit.max()].all()
+        assert (got[v][~odd] == 0.0).all()
+    assert took <= 16.0 * base, (took, base)

@@ -74,7 +74,8 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const __grid_c
                                    rank, S, T, &s_odd, A.err);
   __syncthreads();
   if (s_odd) {
-    sweep_odd<GEOM, G, Q, H, MODEL>(P, sV, A.vol, A.gate_stride, T, v0, v1, u0, u1, band, locks, rank, S, A.err);
+    sweep_odd<GEOM, G, Q, H, MODEL>(P, sV, A.vol, A.gate_stride, T, v0, v1, u0, u1, band, prof, locks, rank, S,
+                                    A.err);
     __syncthreads();
   }
   const int nrow = v1 - v0, ncell = u1 - u0;
