@@ -203,17 +203,20 @@ int trtt_b200_plan3d_backward(trtt_b200_plan3d *plan, const float *sino,
  * an error since the last call, -1 otherwise (flags are cleared). */
 int trtt_b200_plan3d_status(trtt_b200_plan3d *plan, void *stream);
 
-/* Direct-projector kernel selection.  (0, 0): defaults (band kernel with
- * shared-memory accumulation, automatic shape).  band_rows > 0: band kernel
- * with that many detector rows per CTA and `warps` warps per CTA (0 keeps
- * the current value).  band_rows == TRTT_B200_TILES_PULL: closed-form model,
- * atomic-free band kernel (each detector cell accumulated in registers by one
- * owning thread; nu <= 512).  band_rows == TRTT_B200_TILES_TENSOR: closed-form
- * model, band accumulated on the tensor cores (tcgen05 kind::tf32, each
- * value split into two TF32 parts; nu <= 1536, band height chosen from nu).
- * Its accumulation in tensor memory rounds toward zero: about 1.5e-5 relative
- * error at 256^3 -> 512^2 where the default kernels stay below 1e-6, so it is
- * never chosen automatically.  Other band_rows < 0: the per-voxel kernel. */
+/* Direct-projector kernel selection.  (0, 0): defaults (the sweep kernel where
+ * it applies: cubic or tabulated footprint, source and detector plane outside the
+ * volume, at most 8192 table entries between the constant ends; else the band
+ * kernel, automatic shape).  band_rows > 0: band kernel with shared-memory
+ * accumulation, that many detector rows per CTA and `warps` warps per CTA (0
+ * keeps the current value).  A request that is refused (-1) changes nothing.
+ * band_rows == TRTT_B200_TILES_PULL: closed-form model, atomic-free band kernel
+ * (each detector cell accumulated in registers by one owning thread; nu <= 512).
+ * band_rows == TRTT_B200_TILES_TENSOR: closed-form model, band accumulated on the
+ * tensor cores (tcgen05 kind::tf32, each value split into two TF32 parts; nu <=
+ * 1536, band height chosen from nu).  Its accumulation in tensor memory rounds
+ * toward zero: about 1.5e-5 relative error at 256^3 -> 512^2 where the default
+ * kernels stay below 1e-6, so it is never chosen automatically.  Other band_rows
+ * < 0: the per-voxel kernel. */
 #define TRTT_B200_TILES_PULL (-2)
 #define TRTT_B200_TILES_TENSOR (-3)
 
@@ -283,11 +286,10 @@ int trtt_b200_plan3d_factorized(const trtt_b200_plan3d *plan);
  * quads found (all-zero when the group kernels never apply to the plan).
  * set_symmetry(plan, 0) returns to the per-view kernels (results equal to
  * FP32 summation order); 2 (default) uses the group kernels with the member
- * profiles and bands of the direct projector interleaved per detector cell,
- * profiles updated by plain shared-memory loads and stores wherever the
- * voxels' first cells strictly increase along a column and band rows under
- * row locks (35.7 ms per 360 views at 256^3 -> 512^2); 1 the group kernels
- * with one profile per member and shared-memory atomics (87 ms). */
+ * profiles and bands of the direct projector interleaved per detector cell:
+ * the sweep kernel (31.6 ms per 360 views at 256^3 -> 512^2), or with a shape
+ * asked for below k_fwd3d_group (35.7 ms); 1 k_fwd3d_group with one profile per
+ * member and shared-memory atomics (87 ms). */
 int trtt_b200_plan3d_groups(const trtt_b200_plan3d *plan, long *counts);
 int trtt_b200_plan3d_set_symmetry(trtt_b200_plan3d *plan, int on);
 

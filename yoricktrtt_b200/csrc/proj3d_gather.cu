@@ -17,15 +17,15 @@
 // of a column group and add up in shared memory.  Gated scans: the views come
 // sorted by gates, and the sums of the current two gates are in registers.
 //
-// Bound by instruction issue: 80 % of the slots in the parallel scan below,
-// ALU 44 %, FMA 45 %; the detector images stay in L2.  One walk for two voxels
+// Bound by instruction issue: 76 % of the slots for 90 cone views of 128^3,
+// ALU 32 %, FMA 50 %; the detector images stay in L2.  One walk for two voxels
 // halves the shared memory loads and a row load serves four columns, against
 // one warp per column that walked each voxel for itself.  Measured, before ->
-// after: cone 100 x 92 x 75 voxels x 61 views 1.07 -> 0.354 ms, parallel 97^2
-// x 83 x 75 views 1.04 -> 0.64 ms, one cone view of 128^3 75 -> 36 us, 128^2
+// after: cone 100 x 92 x 75 voxels x 61 views 1.07 -> 0.360 ms, parallel 97^2
+// x 83 x 75 views 1.04 -> 0.66 ms, one cone view of 128^3 87 -> 51 us, 128^2
 // x 64 x 10 gates x 400 views 9.04 -> 5.10 ms.  View groups keep
 // k_back3d_group, whose footprint serves two or four views: at 128^3 x 90
-// views 1.36 ms against 1.67 here, and 1.58 with grouped columns in this form;
+// views 1.35 ms against 1.74 here, and 1.58 with grouped columns in this form;
 // at 256^3 x 360 views 35.6 ms against 56.6 with grouped columns in this form.
 #include <cuda_runtime.h>
 
@@ -722,7 +722,8 @@ bool gather_fits(const Params3D &P, const SweepBounds &b)
     return b.rows > 0 && table_slots(P) <= kTableSlots && (P.nz + 1) / 2 / kH < 65535 &&
            table_bytes(P) + GatherRec<MODEL_TABLE>::warps * gather_warp_bytes<MODEL_TABLE>(cap) <= 227 * 1024;
   // (the last test: a walk over two voxels' cells fits the zeros beside a profile,
-  // voxels of up to about 2.4 cells on the detector)
+  // voxels of up to about 2.4 cells on the detector; 60 views of 64^3, voxels of 2.33
+  // cells 0.45 ms, of 2.47 cells 0.61 in the column kernel)
   return b.rows > 0 && GatherRec<MODEL_CUBIC>::warps * gather_warp_bytes<MODEL_CUBIC>(cap) <= 113 * 1024 &&
          (P.nz + 1) / 2 / kH < 65535 && 2.0 * b.hsu + b.du + 4.0 < 2.0 * kSweepGuard - 16.0;
 }

@@ -5,16 +5,17 @@
 //
 // Measured (B200; the band kernel of proj3d_fast.cu, for groups the kernel of
 // proj3d_group.cu before):
-//   61 irregular cone views, 100 x 92 x 75 -> 151 x 133      1.60 -> 0.48 ms
-//   75 parallel views, dense 97 x 97 x 83 -> 129 x 141       2.12 -> 0.74 ms
-//   one cone view, 128^3 -> 256^2 (8 CTAs before)            1.49 -> 0.09 ms
-//   347 gated cone views, 128 x 128 x 64 -> 256^2            8.4 -> 6.6 ms
-//   45 half-turn pairs of views, dense 128^3 -> 256^2        3.08 -> 2.09 ms
-//   90 quads of views, 256^3 -> 512^2 (51% zero voxels)      35.8 -> 31.9 ms
-// Bounds (ncu): pairs and quads shared-memory wavefronts (62% of peak for the
+//   61 irregular cone views, 100 x 92 x 75 -> 151 x 133      1.60 -> 0.50 ms
+//   75 parallel views, dense 97 x 97 x 83 -> 129 x 141       2.14 -> 0.81 ms
+//   one cone view, 128^3 -> 256^2 (8 CTAs before)            1.48 -> 0.08 ms
+//   347 gated cone views, 128 x 128 x 64 -> 256^2 (phantom)  8.0 -> 4.1 ms
+//   45 half-turn pairs of views, dense 128^3 -> 256^2        3.03 -> 2.11 ms
+//   90 quads of views, 256^3 -> 512^2 (51% zero voxels)      35.8 -> 31.8 ms
+// Bounds (ncu): pairs and quads shared-memory wavefronts (66% of peak for the
 // pairs: half of them the band rows, the rest the walks, a quarter of those
-// bank conflicts) at 60% of the issue slots; single views the latencies of
-// their walks and of the row locks at 55% of the issue slots.
+// bank conflicts) at 60% of the issue slots; single views of 128^3 issue (76% of
+// the slots), of smaller volumes the latencies of their walks and of the row locks
+// (the 61 irregular views 55%).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -61,7 +62,8 @@ __global__ void __launch_bounds__(32 * WARPS, MINB) k_fwd3d_sweep(const __grid_c
   int *locks = reinterpret_cast<int *>(base + sizeof(float) * (size_t)rows * US + WARPS * WB);
   if (threadIdx.x < (int)(sizeof(View3D) / 8))
     reinterpret_cast<double *>(&sV)[threadIdx.x] =
-        reinterpret_cast<const double *>(A.views + (A.groups ? A.groups[4 * blockIdx.y] : (int)blockIdx.y))[threadIdx.x];
+        reinterpret_cast<const double *>(
+            A.views + (A.groups ? A.groups[4 * blockIdx.y] : (int)blockIdx.y))[threadIdx.x];
   if (threadIdx.x == 0) {
     s_next = 0;
     s_odd = 0;

@@ -163,7 +163,8 @@ template <> struct SweepRec<MODEL_TABLE> {
 template <int G, int Q, int H, int MODEL> __host__ __device__ constexpr size_t sweep_warp_bytes()
 {
   constexpr int NC = 32 / H;
-  return SweepRec<MODEL>::batch * sizeof(typename SweepRec<MODEL>::T) + sizeof(float2) * kSweepRows * kSweepGroups * NC +
+  return SweepRec<MODEL>::batch * sizeof(typename SweepRec<MODEL>::T) +
+         sizeof(float2) * kSweepRows * kSweepGroups * NC +
          sizeof(float) * (size_t)(NC * (64 * Q + G * kSweepGuard) + G * kSweepGuard);
 }
 __host__ __device__ constexpr int sweep_groups(int R) { return (R + kSweepRows - 1) / kSweepRows; }
@@ -677,7 +678,8 @@ __device__ __forceinline__ void sweep_item(const Params3D &P, const View3D &V, c
             for (int k = 0; k < ng; ++k) {
               int *lock = locks + (gb + k) * NS + s;
               if (!row_lock(lock, err)) continue;
-              float2 *br = reinterpret_cast<float2 *>(band) + (size_t)(gb + k) * kSweepRows * (32 * Q) + lane + 32 * s * SP;
+              float2 *br =
+                  reinterpret_cast<float2 *>(band) + (size_t)(gb + k) * kSweepRows * (32 * Q) + lane + 32 * s * SP;
               float2 sum[kSweepRows][SP];
 #pragma unroll
               for (int rr = 0; rr < kSweepRows; ++rr)

@@ -12,11 +12,11 @@
 // about 5 passes there and about 10 in L1.
 //
 // Measured, 128^3 -> 256^2, 90 cone views, 10001 entries, before (the band and
-// column kernels of proj3d_fast.cu) -> after: direct 7.87 -> 3.08 ms, transpose
-// (dense data) 4.64 -> 3.37 ms.  Bounds: direct the latency of the FP64 chains
-// with 16 warps (49% of the issue slots; the band and the table leave no room
+// column kernels of proj3d_fast.cu) -> after: direct 7.62 -> 3.09 ms, transpose
+// (dense data) 4.64 -> 3.35 ms.  Bounds: direct the latency of the FP64 chains
+// with 16 warps (49% of the issue slots, 61% for a dense volume; the band and the table leave no room
 // for more, 24 warps of 2 columns 2.97 ms); transpose shared-memory wavefronts
-// (63%, over half of them table slots) and issue (62%).
+// (61%, over half of them table slots) and issue (62%).
 #pragma once
 
 #include "fast3d_items.cuh"
@@ -49,7 +49,9 @@ __host__ __device__ __forceinline__ size_t table_bytes(const Params3D &P)
 {
   return P.model == MODEL_TABLE ? sizeof(double) * (size_t)((table_slots(P) + 1) & ~1) : 0;
 }
-constexpr int kTableSlots = 8192;  // largest table range the kernels take
+// Largest table range the kernels take.  90 cone views of a dense 128^3: 8001 slots
+// (a table of 16001 entries) 5.6 + 3.4 ms, 8501 in the general kernels 8.9 + 4.2.
+constexpr int kTableSlots = 8192;
 
 // All threads of the CTA; the caller synchronises.
 __device__ __forceinline__ void table_load(const Params3D &P, double *sh, TableSh &T)
